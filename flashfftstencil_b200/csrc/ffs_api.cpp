@@ -140,6 +140,9 @@ ffs_status prepare_device(int dev)
     CUDA_TRY(prepare_fft3d32());
     CUDA_TRY(prepare_fft2d128());
     CUDA_TRY(prepare_fft1d());
+    CUDA_TRY(prepare_wide());
+    CUDA_TRY(prepare_march());
+    CUDA_TRY(prepare_step());
     CUDA_TRY(prepare_dmma1d());
     CUDA_TRY(prepare_dmma3d());
     CUDA_TRY(prepare_tc2d());
@@ -173,6 +176,10 @@ struct ffs_plan {
         double2 *spec = nullptr;
         BandBox *boxes = nullptr;
     } dev[2];
+    // wide tiles: a chunk's packed rows, and the twiddles per axis
+    double2 *d_wide = nullptr;
+    double2 *d_wtw[3] = {nullptr, nullptr, nullptr};
+    double *d_frame = nullptr; // two buffers of the band's frame
     // tracing (ffs_plan_profile): events bracketing each launch, kind 0 = tile, 1 = band
     struct Mark {
         cudaEvent_t a, b;
@@ -394,6 +401,10 @@ static void release(ffs_plan *p)
     cudaFree(p->d_taps);
     cudaFree(p->d_status);
     cudaFree(p->d_work);
+    cudaFree(p->d_wide);
+    cudaFree(p->d_frame);
+    for (double2 *tw : p->d_wtw)
+        cudaFree(tw);
     for (auto &d : p->dev) {
         cudaFree(d.spec);
         cudaFree(d.boxes);
@@ -413,14 +424,63 @@ static cudaError_t upload(T **dst, const std::vector<T> &src)
     return cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
 }
 
+// Twiddles, workspace and spectra of a wide-tile plan.
+static cudaError_t wide_setup(ffs_plan *p)
+{
+    const PlanSpec &sp = p->spec;
+    cudaError_t e = cudaSuccess;
+    double2 *roots[3] = {nullptr, nullptr, nullptr};
+    for (int d = 0; d < sp.dim && e == cudaSuccess; ++d) {
+        e = upload(&p->d_wtw[d], wide_twiddles(sp.wtile[d], d));
+        if (e == cudaSuccess)
+            e = upload(&roots[d], wide_roots(sp.wtile[d]));
+    }
+    if (e == cudaSuccess && sp.frame)
+        e = cudaMalloc(&p->d_frame, 2 * frame_cells(sp, sp.pass[0].tau) * sizeof(double));
+    if (e == cudaSuccess)
+        e = cudaMalloc(&p->d_wide, (size_t)sp.wchunk * wide_tile_bytes(sp.wtile));
+    for (int k = 0; k < sp.npass_kinds && e == cudaSuccess; ++k) {
+        e = cudaMalloc(&p->dev[k].spec, wide_spectrum_count(sp.wtile) * sizeof(double2));
+        if (e != cudaSuccess)
+            break;
+        WideSpectrum w{};
+        w.out = p->dev[k].spec;
+        w.weights = p->d_weights;
+        w.dim = sp.dim;
+        w.r = sp.radius;
+        w.tau = sp.pass[k].tau;
+        w.scale = 0.5; // the columns are twice the half spectra
+        for (int d = 0; d < 3; ++d) {
+            w.roots[d] = roots[d];
+            w.tile[d] = sp.wtile[d];
+            w.scale /= sp.wtile[d];
+        }
+        e = launch_wide_spectrum(w, nullptr);
+    }
+    if (e == cudaSuccess) // plans run on any stream, also ones that do not wait for this one
+        e = cudaStreamSynchronize(nullptr);
+    for (double2 *r : roots)
+        cudaFree(r);
+    return e;
+}
+
+static ffs_status create_plan(ffs_plan **out, const ffs_problem *problem, Route route);
+
 extern "C" ffs_status ffs_plan_create(ffs_plan **out, const ffs_problem *problem)
 {
     if (!out || !problem)
         return fail(FFS_ERR_INVALID_ARGUMENT, "ffs_plan_create: null argument");
+    const ffs_status st = create_plan(out, problem, kRouteAuto);
+    // wide tiles need a spectrum and a workspace that the one-SM tiles do not
+    return st == FFS_ERR_OUT_OF_MEMORY ? create_plan(out, problem, kRouteNoWide) : st;
+}
+
+static ffs_status create_plan(ffs_plan **out, const ffs_problem *problem, Route route)
+{
     *out = nullptr;
     PlanSpec spec;
     std::string why;
-    ffs_status st = build_plan_spec(*problem, &spec, &why);
+    ffs_status st = build_plan_spec(*problem, &spec, &why, true, route);
     if (st != FFS_OK)
         return fail(st, "%s", why.c_str());
 
@@ -454,6 +514,8 @@ extern "C" ffs_status ffs_plan_create(ffs_plan **out, const ffs_problem *problem
         if ((e = upload(&p->dev[i].boxes, p->spec.pass[i].boxes)) != cudaSuccess)
             return bail(e, "band boxes");
     }
+    if (p->spec.wide && (e = wide_setup(p)) != cudaSuccess)
+        return bail(e, "wide tiles");
     if ((e = cudaMalloc(&p->d_status, sizeof(int))) != cudaSuccess)
         return bail(e, "status word");
     if ((e = cudaMemset(p->d_status, 0, sizeof(int))) != cudaSuccess)
@@ -548,11 +610,132 @@ static BandWork band_work(const ffs_plan *p, int kind, const double *src, double
 static bool band_goes_first(const ffs_plan *p, const PassSpec &ps)
 {
     const PlanSpec &sp = p->spec;
-    if (sp.form != FFS_FORM_FP64_FFT || sp.dim == 1 || (sp.dim == 3 && sp.tile == 32))
+    if (sp.form != FFS_FORM_FP64_FFT || sp.dim == 1 || sp.wide || (sp.dim == 3 && sp.tile == 32))
         return true;
     const int64_t slots = sp.dim == 2 ? std::min<int64_t>(ps.nitems, p->num_sms) : fft3d_grid(ps.nitems, p->num_sms);
     const int64_t tail = ps.nitems % slots;
     return tail == 0 || tail * 10 >= slots * 9;
+}
+
+static WideWork wide_work(const ffs_plan *p, int kind, const double *src, double *dst)
+{
+    const PlanSpec &sp = p->spec;
+    const PassSpec &ps = sp.pass[kind];
+    WideWork w{};
+    w.in = src;
+    w.out = dst;
+    w.work = p->d_wide;
+    w.spec = p->dev[kind].spec;
+    for (int d = 0; d < 3; ++d) {
+        w.tw[d] = p->d_wtw[d];
+        w.n[d] = sp.n[d];
+        w.org[d] = ps.worg[d];
+        w.useful[d] = ps.wuseful[d];
+        w.vhi[d] = ps.vhi[d];
+        w.nt[d] = ps.wnt[d];
+        w.tile[d] = sp.wtile[d];
+        w.halo[d] = ps.whalo[d];
+    }
+    w.periodic = sp.boundary == FFS_BOUNDARY_PERIODIC;
+    return w;
+}
+
+// Taps and the stepped cells of a 2-D plan's direct steps.
+static MarchWork march_work(const ffs_plan *p)
+{
+    const PlanSpec &sp = p->spec;
+    MarchWork m{};
+    std::copy(sp.weights.begin(), sp.weights.end(), m.w);
+    m.nx = (int)sp.n[0];
+    m.ny = (int)sp.n[1];
+    m.periodic = sp.boundary == FFS_BOUNDARY_PERIODIC;
+    const int r = sp.radius, far = 1 << 30; // an open face has no ring
+    m.rx0 = sp.open_faces & 1 ? -far : r;
+    m.rx1 = sp.open_faces & 2 ? far : m.nx - r;
+    m.ry0 = sp.open_faces & 4 ? -far : r;
+    m.ry1 = sp.open_faces & 8 ? far : m.ny - r;
+    return m;
+}
+
+// `tau` direct steps of the whole grid.
+static cudaError_t direct_pass(const ffs_plan *p, int tau, const double *src, double *dst, cudaStream_t s)
+{
+    MarchWork m = march_work(p);
+    m.nregions = 1;
+    m.reg[0] = MarchRegion{src, dst, m.nx, m.nx, 0, m.nx, 0, m.ny, 0, m.nx, 0, m.ny, 0, 0, 0};
+    if (p->spec.blocks) {
+        step_tiles(&m, p->spec.radius, tau);
+        return launch_step2d(m, p->spec.radius, p->spec.star, tau, s);
+    }
+    march_units(&m, p->spec.radius, p->spec.star, tau, p->num_sms);
+    return launch_march2d(m, p->spec.radius, p->spec.star, tau, s);
+}
+
+// The band of a wide pass (the cells within b = r tau of a fixed face) by direct steps on the
+// strips along the faces.  With `left` steps to go, a strip must be right b + r * left deep: each
+// launch reads what the previous one wrote and writes a shallower strip, the first reads the
+// pass's input, the last writes the band itself.
+static cudaError_t frame_pass(const ffs_plan *p, int kind, const double *src, double *dst, cudaStream_t s)
+{
+    const PlanSpec &sp = p->spec;
+    const PassSpec &ps = sp.pass[kind];
+    const int r = sp.radius, tau = ps.tau, most = frame_steps(sp), launches = (tau + most - 1) / most;
+    const int n[2] = {(int)sp.n[0], (int)sp.n[1]};
+    const size_t cells = frame_cells(sp, sp.pass[0].tau);
+    int left = tau;
+    for (int i = 0; i < launches; ++i) {
+        const int steps = split_steps(tau, most, i);
+        const int before = r * (tau + left), after = r * (tau + left - steps); // depths read, written
+        left -= steps;
+        MarchWork m = march_work(p);
+        for (int f = 0; f < 4; ++f) {
+            const int d = f / 2, high = f & 1;
+            if (sp.open_faces >> f & 1)
+                continue;
+            MarchRegion &g = m.reg[m.nregions++];
+            // readable and written boxes, [axis][lo, hi)
+            int rd[2][2] = {{0, n[0]}, {0, n[1]}}, wr[2][2] = {{0, n[0]}, {0, n[1]}};
+            rd[d][0] = high ? std::max(n[d] - before, 0) : 0;
+            rd[d][1] = high ? n[d] : std::min(before, n[d]);
+            wr[d][0] = high ? std::max(n[d] - after, 0) : 0;
+            wr[d][1] = high ? n[d] : std::min(after, n[d]);
+            if (left == 0) // the band: cells outside the exact window, each once (y faces first)
+                for (int a = 0; a < 2; ++a) {
+                    const int lo = (int)ps.vlo[a], hi = (int)ps.vhi[a];
+                    if (a == d) {
+                        wr[a][0] = high ? hi : 0;
+                        wr[a][1] = high ? n[a] : lo;
+                    } else if (a > d) {
+                        wr[a][0] = lo;
+                        wr[a][1] = hi;
+                    }
+                }
+            // strip buffer: 2 b deep along d, the whole other axis
+            const int depth = (int)std::min<int64_t>(2ll * r * sp.pass[0].tau, n[d]);
+            const int64_t pitch = d == 0 ? depth : n[0];
+            const int64_t org = high ? (d == 0 ? n[0] - depth : (int64_t)(n[1] - depth) * pitch) : 0;
+            double *buf = p->d_frame + frame_cells(sp, sp.pass[0].tau, f) - org;
+            g.src = i == 0 ? src : buf + (i & 1 ? 0 : cells);
+            g.spitch = i == 0 ? n[0] : pitch;
+            g.dst = left == 0 ? dst : buf + (i & 1 ? cells : 0);
+            g.dpitch = left == 0 ? n[0] : pitch;
+            g.sx0 = rd[0][0];
+            g.sx1 = rd[0][1];
+            g.sy0 = rd[1][0];
+            g.sy1 = rd[1][1];
+            g.ox0 = wr[0][0];
+            g.ox1 = wr[0][1];
+            g.oy0 = wr[1][0];
+            g.oy1 = wr[1][1];
+            if (g.ox1 <= g.ox0 || g.oy1 <= g.oy0)
+                --m.nregions;
+        }
+        step_tiles(&m, r, steps);
+        const cudaError_t e = launch_step2d(m, r, sp.star, steps, s);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 // One fused pass src -> dst with the pass kind's tau.
@@ -562,19 +745,30 @@ static ffs_status run_pass(const ffs_plan *p, int kind, const double *src, doubl
 {
     const PlanSpec &sp = p->spec;
     const PassSpec &ps = sp.pass[kind];
-    const bool fork = ps.nitems > 0 && !ps.boxes.empty();
+    if (sp.direct) {
+        LaunchMark mark(p, s, 0);
+        const cudaError_t e = direct_pass(p, ps.tau, src, dst, s);
+        return e == cudaSuccess ? FFS_OK : fail(FFS_ERR_CUDA, "direct stepping launch: %s", cudaGetErrorString(e));
+    }
+    const bool has_band = sp.frame || !ps.boxes.empty();
+    const bool fork = ps.nitems > 0 && has_band;
     if (fork) {
         CUDA_TRY(cudaEventRecord(p->ev_fork, s));
         CUDA_TRY(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
     }
     auto band = [&]() -> ffs_status {
-        if (ps.boxes.empty())
+        if (!has_band)
             return FFS_OK;
-        BandWork b = band_work(p, kind, src, dst);
         cudaStream_t bs = fork ? p->side : s;
         {
             LaunchMark mark(p, bs, 1);
-            cudaError_t e = launch_band(b, band_smem_bytes(ps.band_max_vol, b.ntaps), bs);
+            cudaError_t e;
+            if (sp.frame) {
+                e = frame_pass(p, kind, src, dst, bs);
+            } else {
+                BandWork b = band_work(p, kind, src, dst);
+                e = launch_band(b, band_smem_bytes(ps.band_max_vol, b.ntaps), bs);
+            }
             if (e != cudaSuccess)
                 return fail(FFS_ERR_CUDA, "band kernel launch: %s", cudaGetErrorString(e));
         }
@@ -593,7 +787,9 @@ static ffs_status run_pass(const ffs_plan *p, int kind, const double *src, doubl
         const int grid = (int)std::min<int64_t>(ps.nitems, p->num_sms);
         cudaError_t e = cudaSuccess;
         LaunchMark mark(p, s, 0);
-        if (sp.dim == 2 && sp.form == FFS_FORM_FP64_DMMA) {
+        if (sp.wide) {
+            e = launch_wide(wide_work(p, kind, src, dst), ps.nitems, sp.wchunk, s);
+        } else if (sp.dim == 2 && sp.form == FFS_FORM_FP64_DMMA) {
             CUtensorMap tm;
             w.use_tma = make_tmap_2d(&tm, src, sp.n[0], sp.n[1], dmma2d_tile());
             e = launch_dmma2d(w.use_tma ? &tm : nullptr, w, grid, s);
@@ -1191,6 +1387,21 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
     cudaEventCreate(&e1);
     double best = 1e300;
     int arg = 0, arg_tile = 0;
+    // best of three timed executions after a warm-up; the plan is destroyed
+    auto time_plan = [&](ffs_plan *p) {
+        execute_impl(p, din, dout, stream, false);
+        float ms = 0.f, mn = 1e30f;
+        for (int rep = 0; rep < 3; ++rep) {
+            cudaEventRecord(e0, s);
+            execute_impl(p, din, dout, stream, false);
+            cudaEventRecord(e1, s);
+            cudaEventSynchronize(e1);
+            cudaEventElapsedTime(&ms, e0, e1);
+            mn = std::min(mn, ms);
+        }
+        ffs_plan_destroy(p);
+        return mn;
+    };
     for (int tile : tiles) {
         ffs_problem base = *problem;
         base.tile = tile;
@@ -1202,17 +1413,7 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
             ffs_plan *p = nullptr;
             if (ffs_plan_create(&p, &q) != FFS_OK)
                 continue;
-            execute_impl(p, din, dout, stream, false); // warm-up
-            float ms = 0.f, mn = 1e30f;
-            for (int rep = 0; rep < 3; ++rep) {
-                cudaEventRecord(e0, s);
-                execute_impl(p, din, dout, stream, false);
-                cudaEventRecord(e1, s);
-                cudaEventSynchronize(e1);
-                cudaEventElapsedTime(&ms, e0, e1);
-                mn = std::min(mn, ms);
-            }
-            ffs_plan_destroy(p);
+            const float mn = time_plan(p);
             if (mn < tile_best) {
                 tile_best = mn;
                 tile_arg = tau;
@@ -1227,6 +1428,20 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
             arg_tile = at.tile;
         }
     }
+    // the model's choice of wide tile, and of direct stepping, against the best edge
+    if (tiles.size() > 1 && problem->tau == 0)
+        for (Route route : {kRouteWide, kRouteDirect}) {
+            ffs_plan *p = nullptr;
+            if (create_plan(&p, problem, route) != FFS_OK)
+                continue;
+            const int tau = p->spec.tau;
+            const float mn = time_plan(p);
+            if (mn < best) {
+                best = mn;
+                arg = tau;
+                arg_tile = route == kRouteWide ? kWideTuned : kDirectTuned;
+            }
+        }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (!arg) {

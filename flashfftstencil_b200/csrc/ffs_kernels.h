@@ -61,6 +61,36 @@ cudaError_t prepare_fft3d32();
 cudaError_t launch_fft3d32(const TileWork &w, int num_sms, cudaStream_t s);
 size_t fft3d32_smem_bytes();
 
+// FP64 butterfly form on wide tiles (256 .. 2048 cells per axis): three kernels per chunk of
+// tiles over a workspace (ffs_wide.cu).  Tile i covers grid cells from org + (i per axis) *
+// useful; its useful cells start `halo` cells in and are stored below vhi.
+struct WideWork {
+    const double *in;
+    double *out;
+    double2 *work;        // `chunk` tiles of packed rows
+    const double2 *spec;  // S^tau / (2 Nx Ny Nz), [kz][ky][kx], kx padded to Nx / 2 + 16
+    const double2 *tw[3]; // per axis: w_N^(m k1), then w_(N/16)^(m2 k2)
+    int64_t n[3], org[3], useful[3], vhi[3], nt[3];
+    int64_t tile0;        // first tile of the chunk
+    int ntiles;           // tiles of the chunk
+    int tile[3], halo[3];
+    int periodic;
+};
+struct WideSpectrum {
+    double2 *out;
+    const double *weights;
+    const double2 *roots[3]; // exp(+2 pi i m / n) per axis, {re hi, re lo}, {im hi, im lo}
+    int dim, r, tau;
+    int tile[3];
+    double scale;
+};
+int wide_points(int n, int axis); // points per thread of a line of n (axis 0: rows, else columns)
+cudaError_t prepare_wide();
+cudaError_t launch_wide(const WideWork &w, int64_t tiles, int chunk, cudaStream_t s);
+size_t wide_tile_bytes(const int tile[3]);
+size_t wide_spectrum_count(const int tile[3]);
+cudaError_t launch_wide_spectrum(const WideSpectrum &p, cudaStream_t s);
+
 // 1D FP64 butterfly form (four-step DFT-4096 of radix-8 lines).
 cudaError_t prepare_fft1d();
 cudaError_t launch_fft1d(const TileWork &w, int grid, cudaStream_t s);
@@ -108,6 +138,39 @@ struct BandWork {
     int warp_rows;         // 2-D 3 x 3 box: most staged widths are multiples of 32, step by warp rows
 };
 cudaError_t prepare_band(size_t max_smem);
+
+// Direct stepping of 2-D regions in registers (ffs_march.cu).  Coordinates are the grid's:
+// src and dst are offset so that src[y * spitch + x] is cell (x, y).
+struct MarchRegion {
+    const double *src;
+    double *dst;
+    int64_t spitch, dpitch;
+    int sx0, sx1, sy0, sy1; // readable cells of src (fixed boundary)
+    int ox0, ox1, oy0, oy1; // cells to write
+    int strips, chunk, first_unit; // set by march_units
+};
+constexpr int kMarchRegions = 12;
+struct MarchWork {
+    MarchRegion reg[kMarchRegions];
+    double w[25]; // dense (2r+1)^2 taps
+    int nregions, units;
+    int nx, ny, periodic;
+    int rx0, rx1, ry0, ry1; // cells that are stepped (fixed boundary); the others keep their value
+};
+cudaError_t prepare_march();
+int march_max_tau(int r, bool star); // most steps of one launch, 0: radius not supported
+int march_warps(int r, bool star, bool fixed, int tau); // resident warps per SM
+int march_width(int r, int tau);     // columns a warp writes
+void march_units(MarchWork *w, int r, bool star, int tau, int num_sms);
+cudaError_t launch_march2d(const MarchWork &w, int r, bool star, int tau, cudaStream_t s);
+
+// The same regions stepped by blocks that hold a 64 x 64 tile in registers (ffs_step.cu): for
+// regions that do not fill the GPU.
+cudaError_t prepare_step();
+int step_max_steps(int r);          // most steps of one launch, 0: radius not supported
+int step_width(int r, int steps);   // cells of a tile's edge that it writes
+void step_tiles(MarchWork *w, int r, int steps);
+cudaError_t launch_step2d(const MarchWork &w, int r, bool star, int steps, cudaStream_t s);
 
 // Autotuner utilities: a seeded uniform [0, 1) fill, and out[0] = max |y - r|,
 // out[1] = max |r| as ordered bit patterns (out zeroed by the caller).

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <string>
 
 namespace ffst {
 
@@ -257,6 +258,22 @@ constexpr double kTile32ClustersPerSm = 33.0 / 148.0;
 // tau 16: 0.251-0.257 ms for 1849 tiles, 12.5 per SM), against 5.8 us for a 64 x 64 pair.
 constexpr double kTile128Seconds = 20e-6;
 
+// Modelled seconds of a pass's band.  Boxes run concurrently, several per SM; a box costs its
+// direct stepping work plus a per-step barrier latency.
+double band_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
+{
+    double box_max = 0.0, box_sum = 0.0;
+    for (const BandBox &b : ps.boxes) {
+        double v = 1.0;
+        for (int e = 0; e < sp.dim; ++e)
+            v *= std::min<double>(b.ext[e] + 2.0 * sp.radius * ps.tau, (double)sp.n[e]);
+        const double bt = v * ps.tau * (double)sp.taps.size() / 60e9 + ps.tau * 0.3e-6;
+        box_max = std::max(box_max, bt);
+        box_sum += bt;
+    }
+    return ps.boxes.empty() ? 0.0 : std::max(box_max, box_sum / (num_sms * 4.0)) + 3e-6;
+}
+
 // Model of one pass in seconds (used to pick tau).  Rough per-form constants;
 // the tile cost is the measured order of one tile pair per SM.
 double pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
@@ -276,20 +293,12 @@ double pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
         tile_pair_s = kTile32PairSeconds;
     if (sp.dim == 2 && sp.tile == 128)
         tile_pair_s = kTile128Seconds;
+    // an odd row length rules TMA out: the 64 x 64 tiles of a 1999 x 2047 grid took 1.95 times as
+    // long with wrapped plain loads, 1.3 times with clipped ones
+    else if (sp.dim == 2 && sp.form == FFS_FORM_FP64_FFT && (sp.n[0] & 1))
+        tile_pair_s *= sp.boundary == FFS_BOUNDARY_PERIODIC ? 1.9 : 1.3;
     const double waves = std::ceil((double)ps.nitems / (cluster ? std::floor(kTile32ClustersPerSm * num_sms) : num_sms));
-    // band boxes run concurrently, several per SM; a box costs its direct
-    // stepping work plus a per-step barrier latency
-    double box_max = 0.0, box_sum = 0.0;
-    for (const BandBox &b : ps.boxes) {
-        double v = 1.0;
-        for (int e = 0; e < sp.dim; ++e)
-            v *= std::min<double>(b.ext[e] + 2.0 * sp.radius * ps.tau, (double)sp.n[e]);
-        const double bt = v * ps.tau * (double)sp.taps.size() / 60e9 + ps.tau * 0.3e-6;
-        box_max = std::max(box_max, bt);
-        box_sum += bt;
-    }
-    const double band = ps.boxes.empty() ? 0.0 : std::max(box_max, box_sum / (num_sms * 4.0)) + 3e-6;
-    return waves * tile_pair_s + band + 4e-6;
+    return waves * tile_pair_s + band_cost(sp, ps, num_sms) + 4e-6;
 }
 
 int max_tau(const PlanSpec &sp)
@@ -373,6 +382,231 @@ int pick_tile(const PlanSpec &sp, int tau_override)
         }
     }
     return best;
+}
+
+// ---- direct stepping ----
+
+// Measured on 4096^2 and 1999 x 2047 grids (tau 1 .. 8, 5 to 25 taps): 9e12 multiply-adds per
+// second of the 18.4e12, strip and chunk margins counted, with three blocks per SM; the fixed
+// boundary's kernels and the deep ones, two per SM, have fewer warps to hide their latency.
+constexpr double kMarchFmaPerSecond = 9e12;
+constexpr double kMarchLaunchSeconds = 5e-6; // launch, first rows
+constexpr double kMarchBytesPerSecond = 5e12;
+constexpr double kMarchRowSeconds = 0.13e-6; // a warp alone: one level of one row
+
+// Modelled seconds of `tau` fused steps of one nx x ny region.
+double march_cost(const PlanSpec &sp, double nx, double ny, int tau)
+{
+    const int r = sp.radius;
+    const bool fixed = sp.boundary == FFS_BOUNDARY_FIXED;
+    const int warps = march_warps(r, sp.star, fixed, tau);
+    const double rate = kMarchFmaPerSecond * (warps == 12 ? (fixed ? 0.85 : 1.0) : (fixed ? 0.65 : 0.85));
+    const double U = march_width(r, tau), h = 2.0 * r * tau;
+    const double strips = std::ceil(nx / U);
+    const double rows = std::min(std::max(strips * ny / (148.0 * warps), 8.0), ny); // march_units
+    const double cells = strips * 128 * ny * (rows + h) / rows;
+    const double latency = (rows + h) * tau * kMarchRowSeconds * (r == 1 ? 1.0 : 1.5);
+    return std::max(std::max(cells * tau * (double)sp.taps.size() / rate, latency),
+                    16.0 * nx * ny / kMarchBytesPerSecond) +
+           kMarchLaunchSeconds;
+}
+
+// One launch of the block kernel: a step of its tiles, one per SM at a time (5 taps 0.85 us,
+// 9 taps 1.05, 25 taps 1.8, measured on 300 x 260).
+double step_cost(const PlanSpec &sp, double tiles, int steps)
+{
+    const double one = (0.6 + 0.05 * (double)sp.taps.size()) * 1e-6;
+    return kMarchLaunchSeconds + steps * one * std::ceil(tiles / 148.0);
+}
+
+// FFS_DIRECT: "0" keeps direct stepping off, "march" or "blocks" takes that kernel wherever it
+// can run.
+std::string direct_override()
+{
+    const char *env = getenv("FFS_DIRECT");
+    return env ? env : "";
+}
+
+// The whole solve stepped directly: fills tau, passes and the kernel, returns seconds.
+double pick_direct(PlanSpec *sp)
+{
+    const int r = sp->radius;
+    if (sp->dim != 2 || march_max_tau(r, sp->star) == 0 || sp->n[0] >= 1 << 30 || sp->n[1] >= 1 << 30)
+        return INFINITY;
+    double best = INFINITY;
+    const std::string only = direct_override();
+    for (bool blocks : {false, true}) {
+        if (only == (blocks ? "march" : "blocks"))
+            continue;
+        const int most = blocks ? step_max_steps(r) : march_max_tau(r, sp->star);
+        const int least = (sp->T + most - 1) / most;
+        for (int passes = least; passes <= std::min(sp->T, 2 * least); ++passes) {
+            const int tau = (sp->T + passes - 1) / passes;
+            const double U = blocks ? step_width(r, tau) : 1;
+            const double c = passes * (blocks ? step_cost(*sp, std::ceil(sp->n[0] / U) * std::ceil(sp->n[1] / U), tau)
+                                              : march_cost(*sp, (double)sp->n[0], (double)sp->n[1], tau));
+            if (c < best) {
+                best = c;
+                sp->blocks = blocks;
+                sp->tau = tau;
+                sp->passes = (sp->T + tau - 1) / tau;
+                sp->tau_last = sp->T - (sp->passes - 1) * tau;
+            }
+        }
+    }
+    return only == "march" || only == "blocks" ? 0.0 : best;
+}
+
+// Modelled seconds of one direct pass.
+double direct_cost(const PlanSpec &sp, int tau)
+{
+    const double U = step_width(sp.radius, tau);
+    return sp.blocks ? step_cost(sp, std::ceil(sp.n[0] / U) * std::ceil(sp.n[1] / U), tau)
+                     : march_cost(sp, (double)sp.n[0], (double)sp.n[1], tau);
+}
+
+// The band of one wide pass, stepped on the frame: its seconds alone, and the share of them in
+// which the whole GPU is busy with it (what the tiles beside it lose).
+double frame_cost(const PlanSpec &sp, int tau, double *busy)
+{
+    *busy = 0.0;
+    if (sp.boundary != FFS_BOUNDARY_FIXED)
+        return 0.0;
+    const int most = frame_steps(sp), n = (tau + most - 1) / most, steps = (tau + n - 1) / n;
+    const double U = step_width(sp.radius, steps), b = sp.radius * tau;
+    const double tiles = 2.0 * ((double)sp.n[0] + (double)sp.n[1]) / U * std::ceil((1.5 * b - sp.radius * steps) / U);
+    const double launch = step_cost(sp, tiles, steps) - kMarchLaunchSeconds;
+    *busy = n * launch * std::min(1.0, tiles / 148.0);
+    return n * (launch + kMarchLaunchSeconds);
+}
+
+// ---- wide tiles ----
+
+constexpr int kWideEdges[] = {256, 512, 1024, 2048};
+// Workspace of one chunk of tiles.  Fewer, larger launches win over a workspace that stays in
+// the 126 MB L2: Box2D25P 8192^2, T = 128, took 2297 / 2213 / 2018 / 1821 us with chunks of
+// 32 / 80 / 160 / 1000 MB, Box2D9P 4096^2 at T = 32 321 / 293 / 280 / 267 us.
+constexpr size_t kWideChunkBytes = (size_t)1 << 30;
+// Seconds per tile point of a pass: both row kernels by the x edge, the column kernel by the
+// y edge (measured on the two grids above), and per kernel its launch and first and last waves.
+double wide_row_seconds(int n) { return n == 256 ? 5.0e-12 : n == 512 ? 5.2e-12 : n == 1024 ? 5.7e-12 : 5.0e-12; }
+double wide_col_seconds(int n) { return n == 256 ? 4.0e-12 : n == 512 ? 4.8e-12 : n == 1024 ? 5.6e-12 : 7.2e-12; }
+constexpr double kWideLaunchSeconds = 4.5e-6;
+
+// FFS_WIDE_TILE: "0" keeps wide tiles off, "512x1024" takes that edge wherever it fits.
+// Returns -1 off, 0 the model's choice, 1 forced.
+int wide_override(int dim, int tile[3])
+{
+    const char *env = getenv("FFS_WIDE_TILE");
+    if (!env || !*env)
+        return 0;
+    int v[3] = {0, 0, 1};
+    const int got = sscanf(env, "%dx%dx%d", &v[0], &v[1], &v[2]);
+    if (got >= 1 && v[0] == 0)
+        return -1;
+    if (got != dim)
+        return 0;
+    for (int d = 0; d < dim; ++d) {
+        if (std::find(std::begin(kWideEdges), std::end(kWideEdges), v[d]) == std::end(kWideEdges))
+            return 0;
+        tile[d] = v[d];
+    }
+    return 1;
+}
+
+// Tiles of one pass over the exact window (vlo, vhi set): as few per axis as cover it, spread
+// evenly.  False when the edge cannot hold the halo.
+bool wide_geometry(const PlanSpec &sp, PassSpec *ps)
+{
+    ps->nitems = 1;
+    for (int d = 0; d < 3; ++d) {
+        ps->whalo[d] = 0;
+        ps->worg[d] = 0;
+        ps->wuseful[d] = ps->wnt[d] = 1;
+        if (d >= sp.dim)
+            continue;
+        const int h = sp.radius * ps->tau;
+        const int64_t u = sp.wtile[d] - 2 * h, w = ps->vhi[d] - ps->vlo[d];
+        if (u < 16 || sp.n[d] < 128) // 128: rows_fwd steps up to 128 cells around a periodic axis at once
+            return false;
+        if (w <= 0) { // no exact window: the band takes the whole grid
+            ps->nitems = 0;
+            return true;
+        }
+        ps->wnt[d] = ceil_div(w, u);
+        ps->wuseful[d] = ceil_div(w, ps->wnt[d]);
+        ps->whalo[d] = h;
+        ps->worg[d] = ps->vlo[d] - h;
+        ps->nitems *= ps->wnt[d];
+    }
+    return true;
+}
+
+int wide_chunk(const PlanSpec &sp, int64_t tiles)
+{
+    const int64_t c = (int64_t)(kWideChunkBytes / wide_tile_bytes(sp.wtile));
+    return (int)std::max<int64_t>(1, std::min(c, tiles));
+}
+
+double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
+{
+    const double pts = (double)sp.wtile[0] * sp.wtile[1] * sp.wtile[2] * (double)ps.nitems;
+    const double chunks = std::ceil((double)ps.nitems / wide_chunk(sp, ps.nitems));
+    const double tiles = pts * (wide_row_seconds(sp.wtile[0]) + wide_col_seconds(sp.wtile[1])) +
+                         chunks * 3 * kWideLaunchSeconds;
+    // the band runs beside the tiles, but what SMs it holds they do not have (0.7 of that shows:
+    // Box2D9P 1024^2 / 2048^2 / 4096^2 at T = 32 model 50 / 106 / 301 us, measured 46 / 113 / 303)
+    double busy = 0.0;
+    const double band = sp.frame ? frame_cost(sp, ps.tau, &busy) : (busy = band_cost(sp, ps, num_sms));
+    return std::max(tiles + 0.7 * busy, band);
+}
+
+// Fills the wide tile, tau and passes of `sp` with the cheapest modelled choice; returns its
+// seconds (infinite when no wide tile fits).
+double pick_wide(PlanSpec *sp)
+{
+    double best = INFINITY;
+    int forced[3] = {0, 0, 1};
+    const int mode = wide_override(sp->dim, forced);
+    if (sp->form != FFS_FORM_FP64_FFT || sp->dim != 2 || sp->T == 0 || mode < 0)
+        return best;
+    PlanSpec t = *sp;
+    t.wide = true;
+    t.frame = sp->frame = sp->boundary == FFS_BOUNDARY_FIXED && march_max_tau(sp->radius, sp->star) > 0 && sp->n[0] < 1 << 30 &&
+                          sp->n[1] < 1 << 30;
+    for (int passes = 1; passes <= std::min(sp->T, 16); ++passes) {
+        const int tau = (sp->T + passes - 1) / passes;
+        if ((sp->T + tau - 1) / tau != passes)
+            continue;
+        if (2 * round_even(sp->radius * tau) + 16 > 2048)
+            continue;
+        PassSpec ps;
+        t.tile = 2048;
+        geometry(t, tau, &ps);
+        if (!t.frame)
+            band_boxes(t, &ps);
+        if (ps.band_max_vol > 0 && band_smem_bytes(ps.band_max_vol, (int)t.taps.size()) > kBandSmemLimit)
+            continue;
+        for (int ex : kWideEdges)
+            for (int ey : kWideEdges) {
+                if (mode > 0 && (ex != forced[0] || ey != forced[1]))
+                    continue;
+                t.wtile[0] = ex;
+                t.wtile[1] = ey;
+                if (!wide_geometry(t, &ps) || ps.nitems == 0)
+                    continue;
+                const double c = passes * wide_pass_cost(t, ps, 148);
+                if (c < best) {
+                    best = c;
+                    sp->wtile[0] = ex;
+                    sp->wtile[1] = ey;
+                    sp->tau = tau;
+                    sp->passes = passes;
+                    sp->tau_last = sp->T - (passes - 1) * tau;
+                }
+            }
+    }
+    return mode > 0 && best < INFINITY ? 0.0 : best;
 }
 
 void make_spectrum_2d(const PlanSpec &sp, int tau, std::vector<double2> *out)
@@ -521,6 +755,56 @@ void make_spectrum_3d32(const PlanSpec &sp, int tau, std::vector<double2> *out)
                 (*out)[(kz * n + ky) * n + kx] = make_double2((double)(s.re * scale), (double)(s.im * scale));
             }
 }
+
+} // namespace
+
+int frame_steps(const PlanSpec &sp) { return sp.radius == 1 ? 11 : 5; }
+
+size_t frame_cells(const PlanSpec &sp, int tau, int face)
+{
+    size_t at = 0;
+    for (int f = 0; f < face; ++f) { // face 2 d + side: 2 r tau deep along d, the whole other axis
+        const int d = f / 2;
+        if (!(sp.open_faces >> f & 1))
+            at += (size_t)std::min<int64_t>(2ll * sp.radius * tau, sp.n[d]) * sp.n[1 - d];
+    }
+    return at;
+}
+
+std::vector<double2> wide_twiddles(int n, int axis)
+{
+    const int P = wide_points(n, axis), L = n / P;
+    const auto rn = roots(n), rl = roots(L);
+    std::vector<double2> tw(n + L);
+    for (int k1 = 0; k1 < P; ++k1)
+        for (int m = 0; m < L; ++m) {
+            const CLD w = rn[(int64_t)k1 * m % n];
+            tw[k1 * L + m] = make_double2((double)w.re, (double)w.im);
+        }
+    for (int m2 = 0; m2 < L / P; ++m2)
+        for (int k2 = 0; k2 < P; ++k2) {
+            const CLD w = rl[(int64_t)k2 * m2 % L];
+            tw[n + P * m2 + k2] = make_double2((double)w.re, (double)w.im);
+        }
+    return tw;
+}
+
+std::vector<double2> wide_roots(int n)
+{
+    const auto r = roots(n);
+    std::vector<double2> out(2 * (size_t)n);
+    auto split = [](long double v) {
+        const double hi = (double)v;
+        return make_double2(hi, (double)(v - hi));
+    };
+    for (int m = 0; m < n; ++m) {
+        out[2 * m] = split(r[m].re);
+        out[2 * m + 1] = split(-r[m].im); // exp(+2 pi i m / n)
+    }
+    return out;
+}
+
+namespace {
 
 // Byte offset of (row r, K byte kb) in a K-major no-swizzle tcgen05 operand with KB bytes per row.
 size_t operand_offset(int r, int kb, int KB) { return (size_t)(r / 8) * (8 * KB) + (kb / 16) * 128 + (r % 8) * 16 + kb % 16; }
@@ -828,7 +1112,7 @@ std::vector<double> shape_weights(const ShapeDef &sd)
     return w;
 }
 
-ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why, bool with_data)
+ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why, bool with_data, Route route)
 {
     PlanSpec sp;
     auto bad = [&](ffs_status st, const std::string &m) {
@@ -932,6 +1216,9 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
                         sp.taps.push_back(make_int4(dx, dy, dz, idx));
                 }
     }
+    sp.star = sp.dim == 2;
+    for (const int4 &t : sp.taps)
+        sp.star &= t.x == 0 || t.y == 0;
     if (sp.form == FFS_FORM_OZAKI_I8 && sp.slices == 0) { // a calibrated count for this class wins
         const int tuned = tune_lookup(slice_key(sp));
         sp.slices = (tuned >= 4 && tuned <= 8) ? tuned : kDefaultOzakiSlices;
@@ -942,7 +1229,8 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
         return bad(FFS_ERR_UNSUPPORTED, "tile edge not available for this form (1D 4096, 2D 64, 3D 16; the FP64 "
                                         "butterfly form also 128 in 2D and 32 in 3D)");
     sp.tile = p.tile != 0 ? p.tile : fixed_tile;
-    if (p.tile == 0 && alt && sp.T > 0)
+    const bool edge_open = p.tile == 0 && alt && sp.T > 0;
+    if (edge_open)
         sp.tile = pick_tile(sp, p.tau);
     if (sp.T == 0) {
         sp.passes = 0;
@@ -951,7 +1239,40 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
         return FFS_OK;
     }
     pick_tau(&sp, p.tau);
-    if (sp.radius > 0 && sp.tile - 2 * round_even(sp.radius * sp.tau) < 8)
+    // wide tiles and direct stepping: only where the caller left both the edge and the step count
+    // open; a measured choice for the class wins over the model, as for the edges
+    if (edge_open && p.tau == 0) {
+        const int measured = route == kRouteAuto ? tune_lookup(tile_key(sp)) : 0;
+        const bool edge_measured = measured > kDirectTuned; // 64, 128 (2D), 16, 32 (3D)
+        double best = route >= kRouteWide || measured == kWideTuned || measured == kDirectTuned ? INFINITY
+                                                                                              : model_cost(sp, sp.tau);
+        if (edge_measured)
+            best = 0.0;
+        PlanSpec w = sp, d = sp;
+        if (route != kRouteNoWide && route != kRouteDirect && !edge_measured && measured != kDirectTuned) {
+            const double c = pick_wide(&w);
+            if (c < best) {
+                best = c;
+                sp = std::move(w);
+                sp.wide = true;
+                sp.tile = sp.wtile[0];
+            }
+        }
+        // direct stepping is the automatic form's; the butterfly form asked for by name stays that
+        if (p.form == FFS_FORM_AUTO && route != kRouteWide && !edge_measured && measured != kWideTuned &&
+            direct_override() != "0") {
+            const double c = pick_direct(&d);
+            if (c < best) {
+                best = c;
+                sp = std::move(d);
+                sp.direct = true;
+                sp.tile = 128;
+            }
+        }
+    }
+    if ((route == kRouteWide && !sp.wide) || (route == kRouteDirect && !sp.direct))
+        return bad(FFS_ERR_UNSUPPORTED, "no wide tile or direct stepping for this problem");
+    if (!sp.wide && !sp.direct && sp.radius > 0 && sp.tile - 2 * round_even(sp.radius * sp.tau) < 8)
         return bad(FFS_ERR_UNSUPPORTED, "stencil radius too large for the tile");
     sp.npass_kinds = (sp.tau_last != sp.tau) ? 2 : 1;
     sp.last_kind = sp.npass_kinds - 1;
@@ -959,11 +1280,18 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
     for (int k = 0; k < sp.npass_kinds; ++k) {
         const int tau = k == 0 ? sp.tau : sp.tau_last;
         geometry(sp, tau, &sp.pass[k]);
-        band_boxes(sp, &sp.pass[k]);
+        if (sp.wide) {
+            wide_geometry(sp, &sp.pass[k]);
+            sp.wchunk = std::max(sp.wchunk, wide_chunk(sp, sp.pass[k].nitems));
+        }
+        if (sp.direct)
+            sp.pass[k].nitems = 1;
+        else if (!sp.frame)
+            band_boxes(sp, &sp.pass[k]);
         if (sp.pass[k].band_max_vol > 0 &&
             band_smem_bytes(sp.pass[k].band_max_vol, (int)sp.taps.size()) > kBandSmemLimit)
             return bad(FFS_ERR_UNSUPPORTED, "fixed-boundary band does not fit shared memory at this tau");
-        if (with_data) {
+        if (with_data && !sp.wide && !sp.direct) { // (wide tiles: the spectrum is made on the device)
             if (sp.dim == 1 && sp.form == FFS_FORM_FP64_FFT)
                 make_spectrum_1d_half(sp, tau, &sp.pass[k].spectrum);
             else if (sp.dim == 1)
@@ -984,9 +1312,11 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
                 make_spectrum_3d_natural(sp, tau, &sp.pass[k].spectrum);
         }
         const int count = k == 0 ? sp.passes - 1 : 1;
-        sp.est_seconds += (sp.npass_kinds == 1 ? sp.passes : count) * pass_cost(sp, sp.pass[k], 148);
+        sp.est_seconds += (sp.npass_kinds == 1 ? sp.passes : count) *
+                          (sp.direct ? direct_cost(sp, tau)
+                           : sp.wide ? wide_pass_cost(sp, sp.pass[k], 148) : pass_cost(sp, sp.pass[k], 148));
     }
-    if (with_data) {
+    if (with_data && !sp.wide && !sp.direct) {
         make_tables(&sp);
         if (sp.form == FFS_FORM_OZAKI_I8 || sp.form == FFS_FORM_BF16X3) {
             if (sp.dim == 2)
@@ -1024,8 +1354,12 @@ ffs_problem slab_problem(const PlanSpec &sp, int64_t rows, int open)
     q.boundary = sp.boundary;
     q.form = sp.form;
     q.slices = sp.slices;
-    q.tau = sp.tau;
-    q.tile = sp.tile; // the whole grid's tile edge and fused step count
+    if (sp.direct)
+        q.form = FFS_FORM_AUTO; // direct stepping is the automatic form's
+    if (!sp.wide && !sp.direct) { // the whole grid's tile edge and fused step count; a slab of a
+        q.tau = sp.tau; // grid on wide tiles or stepped directly chooses its own
+        q.tile = sp.tile;
+    }
     q.open_faces = open;
     return q;
 }
@@ -1110,7 +1444,7 @@ void fill_plan_info(const PlanSpec &sp, ffs_plan_info *info)
         const PassSpec &ps = sp.pass[0];
         info->halo = ps.halo;
         info->useful = ps.useful;
-        info->tiles = (sp.dim == 2 && sp.tile == 128) ? ps.nitems : ps.nitems * 2;
+        info->tiles = sp.wide || (sp.dim == 2 && sp.tile == 128) ? ps.nitems : ps.nitems * 2;
         const double n = sp.tile;
         // dense DFT-GEMM count: 2 directions x d axes x n^(d+1) complex MACs x 8 flops, per complex tile
         const double dense = 2.0 * sp.dim * std::pow(n, sp.dim + 1) * 8.0;
@@ -1127,7 +1461,20 @@ void fill_plan_info(const PlanSpec &sp, ffs_plan_info *info)
             else // dense DFT-16 GEMMs: 6 stages x (256 lines x 32 x 32) MACs per slice product
                 info->exec_flops_per_pass = 6.0 * 2.0 * 256 * 32 * 32 * products * (double)ps.nitems;
         }
-        if (sp.form == FFS_FORM_FP64_FFT && sp.dim == 1) {
+        if (sp.direct) {
+            info->tiles = 1;
+            info->flops_per_pass = info->exec_flops_per_pass = 2.0 * (double)sp.taps.size() * ps.tau * (double)sp.cells;
+        } else if (sp.wide) {
+            // per line of n points: 16-point butterflies of 176 (log16 n, the last of lower
+            // radix), 15 twiddles of 6 between them; Ny/2 packed rows forward, Nx/2 + 1 columns
+            // both ways, u/2 packed rows back; plus the spectrum product and the packing
+            auto line = [](double e) { return e * (std::log2(e) * 176 / 64 + (e > 256 ? 2 : 1) * 90 / 16.0); };
+            const double nx = sp.wtile[0], ny = sp.wtile[1];
+            info->flops_per_pass = 2.0 * (nx * nx * ny + nx * ny * ny) * 4.0 * (double)ps.nitems;
+            info->exec_flops_per_pass = ((ny + (double)ps.wuseful[1]) / 2 * line(nx) + (nx + 2) * line(ny) +
+                                         10.0 * (nx / 2 + 1) * ny) *
+                                        (double)ps.nitems;
+        } else if (sp.form == FFS_FORM_FP64_FFT && sp.dim == 1) {
             // 256 DFT-64 lines per pair (64 rows, 2 x 64 columns, 64 rows) of 8 x (2 x 56 + 7 x 6),
             // two 4096-point twiddle passes (12 per element: table product and multiply), spectrum
             const double line = 8.0 * (2 * 56 + 7 * 6);

@@ -34,6 +34,10 @@ struct PassSpec {
     int64_t t0[3] = {0, 0, 0}, nt[3] = {1, 1, 1};
     int64_t vlo[3] = {0, 0, 0}, vhi[3] = {1, 1, 1};
     int64_t npx = 0, nitems = 0;
+    // wide tiles (PlanSpec::wide): tile i of an axis covers worg + i * wuseful, its useful
+    // cells start whalo cells in
+    int whalo[3] = {0, 0, 0};
+    int64_t worg[3] = {0, 0, 0}, wuseful[3] = {1, 1, 1}, wnt[3] = {1, 1, 1};
 };
 
 struct PlanSpec {
@@ -48,6 +52,13 @@ struct PlanSpec {
     ffs_form form = FFS_FORM_FP64_DMMA;
     int slices = 0;
     int tile = 0;
+    bool wide = false;           // wide tiles (ffs_wide.cu): `tile` is the x edge
+    int wtile[3] = {1, 1, 1};    // wide tile edges
+    int wchunk = 0;              // tiles per chunk of a wide pass (one workspace)
+    bool direct = false;         // stepped directly, tau steps per pass, no transform:
+    bool blocks = false;         // by blocks (ffs_step.cu), else by marching warps (ffs_march.cu)
+    bool frame = false;          // the wide tiles' band is stepped by ffs_step.cu (no band boxes)
+    bool star = false;           // 2-D: all taps on the axes
     int tau = 0, tau_last = 0, passes = 0;
     int npass_kinds = 0, last_kind = 0;
     PassSpec pass[2];
@@ -56,9 +67,36 @@ struct PlanSpec {
     double est_seconds = 0.0; // autotuner's model estimate for all passes
 };
 
+// Which kernels a plan may use beside its form's one-SM tiles.
+enum Route {
+    kRouteNoWide = 0, // no wide tiles (their workspace did not fit)
+    kRouteAuto = 1,   // the tuning table's or the model's choice
+    kRouteWide = 2,   // only wide tiles (the autotuner's candidates)
+    kRouteDirect = 3, // only direct stepping
+};
 // Validate `p`, pick form/tile/tau and fill `out`.  With `with_data` false the
 // spectra and tables are not computed (fast describe path).
-ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why, bool with_data = true);
+ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why, bool with_data = true,
+                           Route route = kRouteAuto);
+// Values of tile_key's entry for a class whose measured best is not a one-SM tile edge.
+constexpr int kWideTuned = 1, kDirectTuned = 2;
+// Wide tiles: the line transform's twiddles of an axis of n points, and its roots
+// exp(+2 pi i m / n) as pairs of doubles for the spectrum kernel.
+std::vector<double2> wide_twiddles(int n, int axis);
+std::vector<double2> wide_roots(int n);
+
+// Steps of launch `i` of `steps` steps in launches of at most `most`: as even as possible.
+inline int split_steps(int steps, int most, int i)
+{
+    const int n = (steps + most - 1) / most;
+    return steps / n + (i < steps % n ? 1 : 0);
+}
+// Most steps of one launch of the band's frame.  A tile writes 64 - 2 r steps of its 64 cells:
+// Box2D9P 4096^2, T = 32, took 307 / 306 / 297 / 309 us with 4 / 8 / 11 / 16 at a time.
+int frame_steps(const PlanSpec &sp);
+// Doubles of one buffer of the frame (the strips along the fixed faces that the band of a wide
+// pass is stepped on, 2 r tau deep), and the offset of face f (x low, x high, y low, y high).
+size_t frame_cells(const PlanSpec &sp, int tau, int face = 4);
 void fill_plan_info(const PlanSpec &sp, ffs_plan_info *info);
 
 // Model-ranked fusion depths for a problem (best first), at most `count`.

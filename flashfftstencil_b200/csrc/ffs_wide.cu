@@ -1,0 +1,415 @@
+// FP64 butterfly form on wide tiles: one fused pass as three kernels over a workspace.
+//
+// Why: the halo is r tau per side, so the tile edge bounds the fused step count and the
+// share of points that are kept.  A 128 x 128 tile (the largest in one SM's shared memory)
+// keeps (96 / 128)^2 = 0.56 of its points at r tau = 16, and T = 32 needs two such passes; a
+// 512 x 512 tile keeps 0.77 at r tau = 32 in one pass, a 2048 x 2048 one 0.77 at r tau = 128.
+// The price is that the transform leaves the SM between its x and y parts.
+//
+// One tile is Nx x Ny real points, held as Ny / 2 packed complex rows (row y + i row y + Ny/2):
+//   rows_fwd   packed row from the grid, FFT-Nx, stored half by half: Z[j] at slot j and
+//              Z[Nx - j] at slot Hoff + j (j = 0 .. Nx/2, Hoff = Nx/2 + kPad), so that the two
+//              values a column needs lie at the same offset of two aligned segments;
+//   columns    for each kx = j: the true rows' half spectra (Z[j] +- conj Z[Nx-j]) for y and
+//              y + Ny/2, which one thread holds (y = t + L a), FFT-Ny, times S^tau, inverse
+//              FFT-Ny, stored in place: row y's value at slot j (y < Ny/2) or Hoff + j;
+//   rows_inv   two useful rows packed again, inverse FFT-Nx, cropped stores.
+// Every global access of a line's threads is to consecutive addresses, every exchange is
+// conflict-free (ffs_wide.cuh).  Replaces rfft_2d (src/2D/rfft_2d/2d_rfft_1_async.cu:17-364)
+// like the one-SM tiles do.
+#include "ffs_wide.cuh"
+
+#include "ffs_kernels.h"
+
+namespace ffst {
+namespace wide {
+
+constexpr int kRowThreads = 128;
+
+// Points per thread of a row and of a column line, and the threads of a column block.
+constexpr int row_points(int n) { return n <= 512 ? 8 : 16; }
+constexpr int col_points(int n) { return n <= 256 ? 8 : 16; }
+constexpr int col_threads(int n) { return n <= 1024 ? 256 : 512; }
+constexpr int col_blocks_per_sm(int n) { return n <= 256 ? 3 : (n <= 1024 ? 2 : 1); }
+template <int N>
+using RowShape = Shape<N, row_points(N)>;
+template <int N>
+using ColShape = Shape<N, col_points(N)>;
+template <int N>
+constexpr int col_count() { return col_threads(N) / ColShape<N>::L; } // columns side by side in a block
+// row blocks per SM: 64 registers a thread with 8 points, 128 with 16
+constexpr int row_blocks_per_sm(int n) { return 65536 / (row_points(n) == 8 ? 64 : 128) / kRowThreads; }
+
+struct BlockSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <int N>
+struct RowSync {
+    __device__ __forceinline__ void operator()() const
+    {
+        if constexpr (RowShape<N>::L <= 32)
+            __syncwarp();
+        else
+            __syncthreads();
+    }
+};
+
+__device__ __forceinline__ int64_t wrap(int64_t x, int64_t n)
+{
+    const int64_t m = x % n;
+    return m < 0 ? m + n : m;
+}
+
+template <int N>
+__global__ void __launch_bounds__(kRowThreads, row_blocks_per_sm(N)) rows_fwd_kernel(const __grid_constant__ WideWork p)
+{
+    using S = RowShape<N>;
+    extern __shared__ __align__(16) double2 smem[];
+    const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;
+    constexpr int LPB = kRowThreads / S::L;
+    const int half = p.tile[1] >> 1;
+    const int line = blockIdx.x * LPB + l; // Ny / 2 is a multiple of LPB
+    const int tl = line / half, r = line - tl * half;
+    const int64_t tile = p.tile0 + tl;
+    const int64_t ty = tile / p.nt[0], tx = tile - ty * p.nt[0];
+    const int64_t x0 = p.org[0] + tx * p.useful[0] + t, y0 = p.org[1] + ty * p.useful[1] + r;
+    double xr[S::P], xi[S::P];
+    if (p.periodic) {
+        const double *ra = p.in + wrap(y0, p.n[1]) * p.n[0], *rb = p.in + wrap(y0 + half, p.n[1]) * p.n[0];
+        const int nx = (int)p.n[0];
+        int x = (int)wrap(x0, p.n[0]);
+#pragma unroll
+        for (int a = 0; a < S::P; ++a) {
+            xr[a] = __ldg(ra + x);
+            xi[a] = __ldg(rb + x);
+            x += S::L; // L <= 128 <= nx (the plan builder's bound for wide tiles)
+            x -= x >= nx ? nx : 0;
+        }
+    } else {
+        const bool ina = y0 >= 0 && y0 < p.n[1], inb = y0 + half >= 0 && y0 + half < p.n[1];
+        const double *ra = p.in + y0 * p.n[0], *rb = p.in + (y0 + half) * p.n[0];
+#pragma unroll
+        for (int a = 0; a < S::P; ++a) {
+            const int64_t x = x0 + S::L * a;
+            const bool in = x >= 0 && x < p.n[0];
+            xr[a] = in && ina ? __ldg(ra + x) : 0.0;
+            xi[a] = in && inb ? __ldg(rb + x) : 0.0;
+        }
+    }
+    line_fft<N, false, 1, S::P>(xr, xi, t, smem + l * S::SLOTS, p.tw[0], RowSync<N>());
+    constexpr int H = N / 2 + kPad;
+    double2 *w = p.work + (size_t)line * (2 * H);
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int f = t + S::L * a;
+        const double2 v = make_double2(xr[a], xi[a]);
+        if (a < S::P / 2) {
+            w[f] = v;
+            if (a == 0 && t == 0)
+                w[H] = v; // the partner of 0 is 0
+        } else {
+            w[H + N - f] = v;
+            if (a == S::P / 2 && t == 0)
+                w[N / 2] = v; // the partner of N / 2 is N / 2
+        }
+    }
+}
+
+// Columns of a 2D tile: forward, spectrum, inverse.
+template <int N>
+__global__ void __launch_bounds__(col_threads(N), col_blocks_per_sm(N)) cols_kernel(const __grid_constant__ WideWork p)
+{
+    using S = ColShape<N>;
+    constexpr int C = col_count<N>();
+    extern __shared__ __align__(16) double2 smem[];
+    const int c = threadIdx.x % C, t = threadIdx.x / C;
+    const int hx = p.tile[0] >> 1;
+    const int groups = hx / C + 1;
+    const int tl = blockIdx.x / groups, j = (blockIdx.x - tl * groups) * C + c;
+    const bool live = j <= hx;
+    const int H = hx + kPad, P = 2 * H;
+    double2 *w = p.work + (size_t)tl * (N / 2) * P + j;
+    double xr[S::P], xi[S::P];
+    // twice the half spectra of rows y and y + Ny / 2 (the spectrum carries the factor 1/2)
+#pragma unroll
+    for (int a = 0; a < S::P / 2; ++a) {
+        double2 zk = make_double2(0.0, 0.0), zm = zk;
+        if (live) {
+            const double2 *row = w + (t + S::L * a) * P;
+            zk = row[0];
+            zm = row[H];
+        }
+        xr[a] = zk.x + zm.x;
+        xi[a] = zk.y - zm.y;
+        xr[a + S::P / 2] = zk.y + zm.y;
+        xi[a + S::P / 2] = zm.x - zk.x;
+    }
+    line_fft<N, false, C, S::P>(xr, xi, t, smem + c, p.tw[1], BlockSync());
+    const double2 *sp = p.spec + j;
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const double2 s = live ? __ldg(sp + (t + S::L * a) * H) : make_double2(0.0, 0.0);
+        f128::cmul(xr[a], xi[a], s.x, s.y);
+    }
+    __syncthreads(); // the forward transform's last gets before the inverse's first puts
+    line_fft<N, true, C, S::P>(xr, xi, t, smem + c, p.tw[1], BlockSync());
+    const int lo = p.halo[1], hi = p.halo[1] + (int)p.useful[1];
+    if (!live)
+        return;
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int y = t + S::L * a;
+        if (y >= lo && y < hi)
+            w[(t + S::L * (a % (S::P / 2))) * P + (a < S::P / 2 ? 0 : H)] = make_double2(xr[a], xi[a]);
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(kRowThreads, row_blocks_per_sm(N)) rows_inv_kernel(const __grid_constant__ WideWork p)
+{
+    using S = RowShape<N>;
+    extern __shared__ __align__(16) double2 smem[];
+    const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;
+    constexpr int LPB = kRowThreads / S::L;
+    const int half = p.tile[1] >> 1;
+    const int pairs = ((int)p.useful[1] + 1) >> 1;
+    const int ppb = (pairs + LPB - 1) / LPB * LPB; // pairs per tile, rounded to whole blocks
+    const int line = blockIdx.x * LPB + l;
+    const int tl = line / ppb, q = line - tl * ppb;
+    const int64_t tile = p.tile0 + tl;
+    const int64_t ty = tile / p.nt[0], tx = tile - ty * p.nt[0];
+    const int64_t x0 = p.org[0] + tx * p.useful[0] + t, yt = p.org[1] + ty * p.useful[1];
+    const int ya = p.halo[1] + q, yb = ya + pairs;
+    const bool ona = q < pairs && yt + ya < p.vhi[1];
+    const bool onb = ona && yb < p.halo[1] + (int)p.useful[1] && yt + yb < p.vhi[1];
+    if constexpr (S::L <= 32) { // a warp holds whole lines and waits for no other
+        if (__all_sync(0xffffffffu, !ona)) // every lane votes
+            return;
+    }
+    constexpr int H = N / 2 + kPad;
+    const double2 *wt = p.work + (size_t)tl * half * (2 * H);
+    const double2 *wa = wt + (size_t)(ya < half ? ya : ya - half) * (2 * H) + (ya < half ? 0 : H);
+    const double2 *wb = wt + (size_t)(yb < half ? yb : yb - half) * (2 * H) + (yb < half ? 0 : H);
+    double xr[S::P], xi[S::P];
+    const double2 zero = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int f = t + S::L * a;
+        const int j = a < S::P / 2 ? f : N - f;
+        const double2 u = ona ? wa[j] : zero, v = onb ? wb[j] : zero;
+        if (a < S::P / 2) { // A + i B
+            xr[a] = u.x - v.y;
+            xi[a] = u.y + v.x;
+        } else { // conj A + i conj B
+            xr[a] = u.x + v.y;
+            xi[a] = v.x - u.y;
+        }
+    }
+    line_fft<N, true, 1, S::P>(xr, xi, t, smem + l * S::SLOTS, p.tw[0], RowSync<N>());
+    const int lo = p.halo[0], hi = p.halo[0] + (int)p.useful[0];
+    double *oa = p.out + (yt + ya) * p.n[0], *ob = p.out + (yt + yb) * p.n[0];
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int x = t + S::L * a;
+        const int64_t gx = x0 + S::L * a;
+        if (x >= lo && x < hi && gx < p.vhi[0]) {
+            if (ona)
+                oa[gx] = xr[a];
+            if (onb)
+                ob[gx] = xi[a];
+        }
+    }
+}
+
+// ---- the spectrum S^tau, in double-double arithmetic ----
+//
+// S(k)^tau by repeated squaring multiplies the relative error of S by tau, so plain FP64
+// would lose log2(tau) bits where |S| is close to 1.  A double-double pair carries 106
+// bits; the roots come from the host in extended precision.
+
+struct DD {
+    double hi, lo;
+};
+__device__ __forceinline__ DD quick_two_sum(double a, double b)
+{
+    const double s = a + b;
+    return {s, b - (s - a)};
+}
+__device__ __forceinline__ DD dd_add(DD a, DD b)
+{
+    const double s = a.hi + b.hi, v = s - a.hi;
+    const double e = (a.hi - (s - v)) + (b.hi - v);
+    return quick_two_sum(s, e + (a.lo + b.lo));
+}
+__device__ __forceinline__ DD dd_neg(DD a) { return {-a.hi, -a.lo}; }
+__device__ __forceinline__ DD dd_mul(DD a, DD b)
+{
+    const double p = a.hi * b.hi;
+    const double e = fma(a.hi, b.hi, -p) + (a.hi * b.lo + a.lo * b.hi);
+    return quick_two_sum(p, e);
+}
+struct CDD {
+    DD re, im;
+};
+__device__ __forceinline__ CDD cdd_mul(CDD a, CDD b)
+{
+    return {dd_add(dd_mul(a.re, b.re), dd_neg(dd_mul(a.im, b.im))), dd_add(dd_mul(a.re, b.im), dd_mul(a.im, b.re))};
+}
+__device__ __forceinline__ CDD cdd_add(CDD a, CDD b) { return {dd_add(a.re, b.re), dd_add(a.im, b.im)}; }
+
+// roots[m] = exp(+2 pi i m / n) as {re.hi, re.lo}, {im.hi, im.lo}
+__device__ __forceinline__ CDD root_of(const double2 *roots, int n, int d, int k)
+{
+    int m = (int)(((int64_t)d * k) % n);
+    m += m < 0 ? n : 0;
+    const double2 a = __ldg(roots + 2 * m), b = __ldg(roots + 2 * m + 1);
+    return {{a.x, a.y}, {b.x, b.y}};
+}
+
+__global__ void __launch_bounds__(256) spectrum_kernel(const WideSpectrum p)
+{
+    const int H = p.tile[0] / 2 + kPad;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t line = i / H;
+    const int kx = (int)(i - line * H);
+    if (line >= (int64_t)p.tile[1] * p.tile[2])
+        return;
+    if (kx > p.tile[0] / 2) {
+        p.out[i] = make_double2(0.0, 0.0);
+        return;
+    }
+    const int kz = (int)(line / p.tile[1]), ky = (int)(line - (int64_t)kz * p.tile[1]);
+    const int r = p.r, ry = p.dim >= 2 ? r : 0, rz = p.dim >= 3 ? r : 0, K = 2 * r + 1;
+    const DD z0 = {0.0, 0.0};
+    CDD s = {z0, z0};
+    for (int dz = -rz; dz <= rz; ++dz) {
+        CDD plane = {z0, z0};
+        for (int dy = -ry; dy <= ry; ++dy) {
+            CDD row = {z0, z0};
+            for (int dx = -r; dx <= r; ++dx) {
+                const double w = __ldg(p.weights + ((dz + rz) * (2 * ry + 1) + (dy + ry)) * K + (dx + r));
+                if (w != 0.0) {
+                    const CDD e = root_of(p.roots[0], p.tile[0], dx, kx);
+                    const DD wd = {w, 0.0};
+                    row = cdd_add(row, {dd_mul(e.re, wd), dd_mul(e.im, wd)});
+                }
+            }
+            plane = cdd_add(plane, p.dim >= 2 ? cdd_mul(row, root_of(p.roots[1], p.tile[1], dy, ky)) : row);
+        }
+        s = cdd_add(s, p.dim >= 3 ? cdd_mul(plane, root_of(p.roots[2], p.tile[2], dz, kz)) : plane);
+    }
+    CDD v = {{1.0, 0.0}, z0};
+    for (int e = p.tau; e > 0; e >>= 1) {
+        if (e & 1)
+            v = cdd_mul(v, s);
+        s = cdd_mul(s, s);
+    }
+    p.out[i] = make_double2(v.re.hi * p.scale, v.im.hi * p.scale); // scale: a power of two
+}
+
+template <int N>
+cudaError_t prepare_one()
+{
+    const int rows = (int)sizeof(double2) * RowShape<N>::SLOTS * (kRowThreads / RowShape<N>::L);
+    const int cols = (int)sizeof(double2) * ColShape<N>::SLOTS * col_count<N>();
+    cudaError_t e = cudaFuncSetAttribute(rows_fwd_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(rows_inv_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cols_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, cols);
+    return e;
+}
+
+template <int N>
+cudaError_t rows(const WideWork &w, bool inverse, cudaStream_t s)
+{
+    constexpr int LPB = kRowThreads / RowShape<N>::L;
+    const size_t smem = sizeof(double2) * RowShape<N>::SLOTS * LPB;
+    if (!inverse) {
+        rows_fwd_kernel<N><<<(unsigned)((int64_t)w.ntiles * (w.tile[1] / 2) / LPB), kRowThreads, smem, s>>>(w);
+    } else {
+        const int pairs = ((int)w.useful[1] + 1) / 2;
+        const int64_t blocks = (int64_t)w.ntiles * ((pairs + LPB - 1) / LPB);
+        rows_inv_kernel<N><<<(unsigned)blocks, kRowThreads, smem, s>>>(w);
+    }
+    return cudaGetLastError();
+}
+
+template <int N>
+cudaError_t cols(const WideWork &w, cudaStream_t s)
+{
+    constexpr int C = col_count<N>();
+    const size_t smem = sizeof(double2) * ColShape<N>::SLOTS * C;
+    cols_kernel<N><<<(unsigned)(w.ntiles * (w.tile[0] / 2 / C + 1)), col_threads(N), smem, s>>>(w);
+    return cudaGetLastError();
+}
+
+#define FFS_WIDE_BY_EDGE(edge, call)                                                                                \
+    switch (edge) {                                                                                                 \
+    case 256: { constexpr int N = 256; return call; }                                                               \
+    case 512: { constexpr int N = 512; return call; }                                                               \
+    case 1024: { constexpr int N = 1024; return call; }                                                             \
+    case 2048: { constexpr int N = 2048; return call; }                                                             \
+    default: return cudaErrorInvalidValue;                                                                          \
+    }
+
+cudaError_t rows_any(const WideWork &w, bool inverse, cudaStream_t s)
+{
+    FFS_WIDE_BY_EDGE(w.tile[0], (rows<N>(w, inverse, s)))
+}
+cudaError_t cols_any(const WideWork &w, cudaStream_t s)
+{
+    FFS_WIDE_BY_EDGE(w.tile[1], (cols<N>(w, s)))
+}
+
+} // namespace wide
+
+cudaError_t prepare_wide()
+{
+    cudaError_t e = wide::prepare_one<256>();
+    if (e == cudaSuccess)
+        e = wide::prepare_one<512>();
+    if (e == cudaSuccess)
+        e = wide::prepare_one<1024>();
+    if (e == cudaSuccess)
+        e = wide::prepare_one<2048>();
+    return e;
+}
+
+cudaError_t launch_wide(const WideWork &w, int64_t tiles, int chunk, cudaStream_t s)
+{
+    for (int64_t t = 0; t < tiles; t += chunk) {
+        WideWork c = w;
+        c.tile0 = t;
+        c.ntiles = (int)(tiles - t < chunk ? tiles - t : chunk);
+        cudaError_t e = wide::rows_any(c, false, s);
+        if (e == cudaSuccess)
+            e = wide::cols_any(c, s);
+        if (e == cudaSuccess)
+            e = wide::rows_any(c, true, s);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
+int wide_points(int n, int axis) { return axis == 0 ? wide::row_points(n) : wide::col_points(n); }
+
+size_t wide_tile_bytes(const int tile[3]) // workspace of one tile
+{
+    return sizeof(double2) * (size_t)(tile[0] + 2 * wide::kPad) * (tile[1] / 2) * tile[2];
+}
+
+size_t wide_spectrum_count(const int tile[3])
+{
+    return (size_t)(tile[0] / 2 + wide::kPad) * tile[1] * tile[2];
+}
+
+cudaError_t launch_wide_spectrum(const WideSpectrum &p, cudaStream_t s)
+{
+    const int64_t count = (int64_t)wide_spectrum_count(p.tile);
+    wide::spectrum_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+} // namespace ffst

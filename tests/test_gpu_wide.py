@@ -1,0 +1,98 @@
+"""Wide tiles (256 .. 2048 cells per axis, three kernels per pass) against the oracle: every edge in x
+and in y, both boundaries, grids below, at and just past one tile, odd sizes and 8-byte-aligned
+grids, in-place calls, several passes with a shorter last one, and host slabs (open faces)."""
+import numpy as np
+import pytest
+
+import flashfftstencil_b200 as ffs
+import oracle
+from tests.helpers import rel_errors, seeded_grid, seeded_weights
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # the FP64 forms' tolerance
+
+
+def _solve(ext, T, boundary, radius=1, weights=None, form="auto", in_place=False, offset=0):
+    import torch
+    w = seeded_weights(2, radius, 3) if weights is None else weights
+    plan = ffs.Plan(2, None, ext, T, weights=w, radius=radius, boundary=boundary, form=form)
+    x = seeded_grid((ext[1], ext[0]), 4)
+    buf = torch.empty(x.size + offset, dtype=torch.float64, device="cuda")
+    d = buf[offset:].view(x.shape)
+    d.copy_(torch.from_numpy(x))
+    out = d if in_place else torch.full_like(d, float("nan"))
+    plan.run(d, out)
+    torch.cuda.synchronize()
+    ref = oracle.run(x, w, radius, T, oracle.FIXED if boundary == "fixed" else oracle.PERIODIC)
+    return plan, rel_errors(out.cpu().numpy(), ref)[0]
+
+
+@pytest.mark.parametrize("boundary", ["fixed", "periodic"])
+@pytest.mark.parametrize("edge", ["256x256", "512x256", "256x512", "1024x512", "512x1024", "2048x256", "256x2048"])
+def test_every_edge_matches_the_oracle(monkeypatch, edge, boundary):
+    monkeypatch.setenv("FFS_WIDE_TILE", edge)
+    plan, err = _solve((333, 291), 17, boundary)
+    assert plan.info["tile"] == int(edge.split("x")[0]) and plan.info["tau"] == 17
+    assert err <= TOL
+
+
+@pytest.mark.parametrize("boundary", ["fixed", "periodic"])
+@pytest.mark.parametrize("ext,T,radius", [
+    ((128, 128), 5, 1),    # the smallest sides
+    ((226, 226), 15, 1),   # one tile of useful cells, to the cell (periodic)
+    ((227, 453), 15, 1),   # one and two tiles and a cell
+    ((511, 300), 40, 2),   # r tau of 80
+    ((300, 260), 13, 3),   # radius without strip stepping: the band's boxes
+])
+def test_tile_remainders(monkeypatch, ext, T, radius, boundary):
+    monkeypatch.setenv("FFS_WIDE_TILE", "256x256")
+    plan, err = _solve(ext, T, boundary, radius)
+    assert plan.info["tile"] == 256 and err <= TOL
+
+
+@pytest.mark.parametrize("in_place,offset", [(True, 0), (False, 1), (True, 1)])
+@pytest.mark.parametrize("T", [30, 250])  # one pass, several with a shorter last one
+def test_in_place_and_unaligned(monkeypatch, T, in_place, offset):
+    monkeypatch.setenv("FFS_WIDE_TILE", "256x256")
+    plan, err = _solve((301, 277), T, "fixed", in_place=in_place, offset=offset)
+    assert plan.info["tile"] == 256 and err <= TOL
+
+
+@pytest.mark.parametrize("boundary", ["fixed", "periodic"])
+def test_host_slabs_of_a_wide_grid(monkeypatch, boundary):
+    monkeypatch.setenv("FFS_WIDE_TILE", "256x256")
+    monkeypatch.setenv("FFS_HOST_SLABS", "3")
+    w = seeded_weights(2, 1, 5)
+    plan = ffs.Plan(2, None, (320, 900), 20, weights=w, radius=1, boundary=boundary, form="auto")
+    assert plan.info["tile"] == 256 and plan.info["host_slabs"] == 3
+    x = seeded_grid((900, 320), 6)
+    ref = oracle.run(x, w, 1, 20, oracle.FIXED if boundary == "fixed" else oracle.PERIODIC)
+    assert rel_errors(plan.run_host(x), ref)[0] <= TOL
+
+
+def test_signed_weights_and_a_star(monkeypatch):
+    monkeypatch.setenv("FFS_WIDE_TILE", "512x256")
+    w = np.random.default_rng(2).standard_normal((5, 5))
+    w /= np.abs(np.fft.fft2(w, s=(256, 256))).max()
+    assert _solve((400, 350), 24, "periodic", 2, w)[1] <= TOL
+    star = np.zeros((5, 5))
+    star[2] = [0.1, 0.15, 0.3, 0.15, 0.1]
+    star[:, 2] += [0.05, 0.05, 0.0, 0.05, 0.05]
+    assert _solve((400, 350), 24, "fixed", 2, star)[1] <= TOL
+
+
+def test_repeats_use_each_input(monkeypatch):
+    """Calls on alternating buffers share the workspace: each result is its own input's, bit for bit."""
+    import torch
+    monkeypatch.setenv("FFS_WIDE_TILE", "256x256")
+    plan = ffs.Plan(2, "Box2D9P", (300, 300), 20, boundary="fixed", form="auto")
+    xs = [torch.from_numpy(seeded_grid((300, 300), k)).cuda() for k in range(2)]
+    first = [plan.run(x).clone() for x in xs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    outs = [torch.empty_like(x) for x in xs]
+    for _ in range(4):
+        for x, o, s in zip(xs, outs, streams):
+            plan.run(x, o, stream=s)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(first, outs))

@@ -166,6 +166,7 @@ struct ffs_plan {
     PlanSpec spec;            // host description (geometry, spectra, boxes)
     int device = 0;
     int num_sms = 148;
+    unsigned char *d_memory = nullptr; // all of the plan's device memory; the pointers below are into it
     double2 *d_tables = nullptr;
     unsigned char *d_aslices = nullptr;
     double *d_weights = nullptr;
@@ -395,54 +396,60 @@ static void release(ffs_plan *p)
             cudaStreamDestroy(h.s_out);
         release_slabs(h.slabs);
     }
-    cudaFree(p->d_tables);
-    cudaFree(p->d_aslices);
-    cudaFree(p->d_weights);
-    cudaFree(p->d_taps);
-    cudaFree(p->d_status);
-    cudaFree(p->d_work);
-    cudaFree(p->d_wide);
-    cudaFree(p->d_frame);
-    for (double2 *tw : p->d_wtw)
-        cudaFree(tw);
-    for (auto &d : p->dev) {
-        cudaFree(d.spec);
-        cudaFree(d.boxes);
-    }
+    cudaFree(p->d_memory);
     delete p;
 }
 
-template <typename T>
-static cudaError_t upload(T **dst, const std::vector<T> &src)
-{
-    *dst = nullptr;
-    if (src.empty())
-        return cudaSuccess;
-    cudaError_t e = cudaMalloc(dst, src.size() * sizeof(T));
-    if (e != cudaSuccess)
-        return e;
-    return cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
-}
+// A plan's device memory is one allocation, filled by one copy: each cudaMalloc of 1 MB to 180 MB
+// takes 0.4 ms, and a plan has up to a dozen arrays.  Collects the arrays with their contents
+// first (each starts on a 256-byte boundary), then the buffers without.
+struct PlanMemory {
+    struct Piece {
+        void **at;
+        size_t offset;
+    };
+    std::vector<Piece> pieces;
+    std::vector<unsigned char> image;
+    size_t size = 0;
 
-// Twiddles, workspace and spectra of a wide-tile plan.
-static cudaError_t wide_setup(ffs_plan *p)
+    template <typename T>
+    void put(T **at, const std::vector<T> &src)
+    {
+        *at = nullptr;
+        if (src.empty())
+            return;
+        image.resize((image.size() + 255) & ~(size_t)255);
+        pieces.push_back({reinterpret_cast<void **>(at), image.size()});
+        const unsigned char *b = reinterpret_cast<const unsigned char *>(src.data());
+        image.insert(image.end(), b, b + src.size() * sizeof(T));
+        size = image.size();
+    }
+    template <typename T>
+    void reserve(T **at, size_t count) // after the last put
+    {
+        size = (size + 255) & ~(size_t)255;
+        pieces.push_back({reinterpret_cast<void **>(at), size});
+        size += count * sizeof(T);
+    }
+    cudaError_t allocate(unsigned char **base)
+    {
+        cudaError_t e = cudaMalloc(base, size);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(*base, image.data(), image.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess)
+            return e;
+        for (const Piece &q : pieces)
+            *q.at = *base + q.offset;
+        return cudaSuccess;
+    }
+};
+
+// The spectra of a wide-tile plan, made on the device (`roots` per axis, in its memory).
+static cudaError_t wide_spectra(const ffs_plan *p, double2 *const roots[3])
 {
     const PlanSpec &sp = p->spec;
     cudaError_t e = cudaSuccess;
-    double2 *roots[3] = {nullptr, nullptr, nullptr};
-    for (int d = 0; d < sp.dim && e == cudaSuccess; ++d) {
-        e = upload(&p->d_wtw[d], wide_twiddles(sp.wtile[d], d));
-        if (e == cudaSuccess)
-            e = upload(&roots[d], wide_roots(sp.wtile[d]));
-    }
-    if (e == cudaSuccess && sp.frame)
-        e = cudaMalloc(&p->d_frame, 2 * frame_cells(sp, sp.pass[0].tau) * sizeof(double));
-    if (e == cudaSuccess)
-        e = cudaMalloc(&p->d_wide, (size_t)sp.wchunk * wide_tile_bytes(sp.wtile));
     for (int k = 0; k < sp.npass_kinds && e == cudaSuccess; ++k) {
-        e = cudaMalloc(&p->dev[k].spec, wide_spectrum_count(sp.wtile) * sizeof(double2));
-        if (e != cudaSuccess)
-            break;
         WideSpectrum w{};
         w.out = p->dev[k].spec;
         w.weights = p->d_weights;
@@ -459,8 +466,6 @@ static cudaError_t wide_setup(ffs_plan *p)
     }
     if (e == cudaSuccess) // plans run on any stream, also ones that do not wait for this one
         e = cudaStreamSynchronize(nullptr);
-    for (double2 *r : roots)
-        cudaFree(r);
     return e;
 }
 
@@ -500,30 +505,36 @@ static ffs_status create_plan(ffs_plan **out, const ffs_problem *problem, Route 
                     cudaGetErrorString(e));
     };
     cudaError_t e;
-    if ((e = upload(&p->d_tables, p->spec.tables)) != cudaSuccess)
-        return bail(e, "tables");
-    if ((e = upload(&p->d_aslices, p->spec.a_slices)) != cudaSuccess)
-        return bail(e, "tensor-core operand slices");
-    if ((e = upload(&p->d_weights, p->spec.weights)) != cudaSuccess)
-        return bail(e, "weights");
-    if ((e = upload(&p->d_taps, p->spec.taps)) != cudaSuccess)
-        return bail(e, "taps");
-    for (int i = 0; i < p->spec.npass_kinds; ++i) {
-        if ((e = upload(&p->dev[i].spec, p->spec.pass[i].spectrum)) != cudaSuccess)
-            return bail(e, "spectrum");
-        if ((e = upload(&p->dev[i].boxes, p->spec.pass[i].boxes)) != cudaSuccess)
-            return bail(e, "band boxes");
+    const PlanSpec &sp = p->spec;
+    PlanMemory mem;
+    double2 *roots[3] = {nullptr, nullptr, nullptr};
+    mem.put(&p->d_status, std::vector<int>{0});
+    mem.put(&p->d_tables, sp.tables);
+    mem.put(&p->d_aslices, sp.a_slices);
+    mem.put(&p->d_weights, sp.weights);
+    mem.put(&p->d_taps, sp.taps);
+    for (int k = 0; k < sp.npass_kinds; ++k) {
+        mem.put(&p->dev[k].spec, sp.pass[k].spectrum);
+        mem.put(&p->dev[k].boxes, sp.pass[k].boxes);
     }
-    if (p->spec.wide && (e = wide_setup(p)) != cudaSuccess)
-        return bail(e, "wide tiles");
-    if ((e = cudaMalloc(&p->d_status, sizeof(int))) != cudaSuccess)
-        return bail(e, "status word");
-    if ((e = cudaMemset(p->d_status, 0, sizeof(int))) != cudaSuccess)
-        return bail(e, "status word");
-    if (p->spec.passes >= 1) {
-        if ((e = cudaMalloc(&p->d_work, p->spec.cells * sizeof(double))) != cudaSuccess)
-            return bail(e, "workspace");
+    if (sp.wide)
+        for (int d = 0; d < sp.dim; ++d) {
+            mem.put(&p->d_wtw[d], wide_twiddles(sp.wtile[d], d));
+            mem.put(&roots[d], wide_roots(sp.wtile[d]));
+        }
+    if (sp.passes >= 1)
+        mem.reserve(&p->d_work, sp.cells);
+    if (sp.wide) {
+        for (int k = 0; k < sp.npass_kinds; ++k)
+            mem.reserve(&p->dev[k].spec, wide_spectrum_count(sp.wtile));
+        mem.reserve(&p->d_wide, (size_t)sp.wchunk * wide_tile_bytes(sp.wtile) / sizeof(double2));
+        if (sp.frame)
+            mem.reserve(&p->d_frame, 2 * frame_cells(sp, sp.pass[0].tau));
     }
+    if ((e = mem.allocate(&p->d_memory)) != cudaSuccess)
+        return bail(e, "plan memory");
+    if (sp.wide && (e = wide_spectra(p, roots)) != cudaSuccess)
+        return bail(e, "wide tiles' spectrum");
     if ((e = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
@@ -1280,7 +1291,12 @@ extern "C" ffs_status ffs_plan_get_info(const ffs_plan *plan, ffs_plan_info *inf
     if (!plan || !info)
         return fail(FFS_ERR_INVALID_ARGUMENT, "ffs_plan_get_info: null argument");
     fill_plan_info(plan->spec, info);
-    info->work_bytes = plan->d_work ? (int64_t)(plan->spec.cells * sizeof(double)) : 0;
+    const PlanSpec &sp = plan->spec;
+    size_t work = plan->d_work ? sp.cells * sizeof(double) : 0;
+    if (sp.wide)
+        work += (size_t)sp.wchunk * wide_tile_bytes(sp.wtile) +
+                (sp.frame ? 2 * frame_cells(sp, sp.pass[0].tau) * sizeof(double) : 0);
+    info->work_bytes = (int64_t)work;
     return FFS_OK;
 }
 

@@ -143,6 +143,7 @@ ffs_status prepare_device(int dev)
     CUDA_TRY(prepare_wide());
     CUDA_TRY(prepare_march());
     CUDA_TRY(prepare_step());
+    CUDA_TRY(prepare_march3());
     CUDA_TRY(prepare_dmma1d());
     CUDA_TRY(prepare_dmma3d());
     CUDA_TRY(prepare_tc2d());
@@ -668,9 +669,44 @@ static MarchWork march_work(const ffs_plan *p)
     return m;
 }
 
+// The same of a 3-D plan (radius 1).
+static March3Work march3_work(const ffs_plan *p)
+{
+    const PlanSpec &sp = p->spec;
+    March3Work m{};
+    std::copy(sp.weights.begin(), sp.weights.end(), m.w);
+    m.periodic = sp.boundary == FFS_BOUNDARY_PERIODIC;
+    for (int d = 0; d < 3; ++d) {
+        m.n[d] = (int)sp.n[d];
+        m.slo[d] = sp.open_faces >> (2 * d) & 1 ? -(1 << 30) : 1;
+        m.shi[d] = sp.open_faces >> (2 * d + 1) & 1 ? 1 << 30 : m.n[d] - 1;
+    }
+    return m;
+}
+
 // `tau` direct steps of the whole grid.
 static cudaError_t direct_pass(const ffs_plan *p, int tau, const double *src, double *dst, cudaStream_t s)
 {
+    if (p->spec.dim == 1) {
+        const PlanSpec &sp = p->spec;
+        LineWork l{};
+        l.in = src;
+        l.out = dst;
+        std::copy(sp.weights.begin(), sp.weights.end(), l.w);
+        l.n = sp.n[0];
+        l.slo = sp.open_faces & 1 ? INT64_MIN : sp.radius;
+        l.shi = sp.open_faces & 2 ? INT64_MAX : l.n - sp.radius;
+        l.steps = tau;
+        l.periodic = sp.boundary == FFS_BOUNDARY_PERIODIC;
+        return launch_line(l, sp.radius, sp.line_k, s);
+    }
+    if (p->spec.dim == 3) {
+        March3Work m = march3_work(p);
+        m.in = src;
+        m.out = dst;
+        march3_units(&m, (int)p->spec.taps.size(), p->num_sms);
+        return launch_march3d(m, p->spec.star, s);
+    }
     MarchWork m = march_work(p);
     m.nregions = 1;
     m.reg[0] = MarchRegion{src, dst, m.nx, m.nx, 0, m.nx, 0, m.ny, 0, m.nx, 0, m.ny, 0, 0, 0};
@@ -1436,6 +1472,7 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
             }
         }
         PlanSpec at;
+        base.tau = tile_arg; // (with the step count open too, 1-D could name another route)
         if (tile_arg && build_plan_spec(base, &at, &why, false) == FFS_OK)
             tune_record(tune_key(at), tile_arg); // this edge's best step count
         if (tile_arg && tile_best < best) {
@@ -1445,7 +1482,8 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
         }
     }
     // the model's choice of wide tile, and of direct stepping, against the best edge
-    if (tiles.size() > 1 && problem->tau == 0)
+    const bool routes = problem->tile == 0 && problem->tau == 0 && spec.form == FFS_FORM_FP64_FFT;
+    if (routes)
         for (Route route : {kRouteWide, kRouteDirect}) {
             ffs_plan *p = nullptr;
             if (create_plan(&p, problem, route) != FFS_OK)
@@ -1465,7 +1503,7 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
         cudaFree(dout);
         return fail(FFS_ERR_INTERNAL, "ffs_autotune: no candidate could run");
     }
-    if (tiles.size() > 1)
+    if (tiles.size() > 1 || routes)
         tune_record(tile_key(spec), arg_tile);
     if (spec.form == FFS_FORM_OZAKI_I8 && problem->slices == 0) {
         // the slice count at the chosen fused step count, recorded with that count

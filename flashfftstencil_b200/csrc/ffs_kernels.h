@@ -172,6 +172,31 @@ int step_width(int r, int steps);   // cells of a tile's edge that it writes
 void step_tiles(MarchWork *w, int r, int steps);
 cudaError_t launch_step2d(const MarchWork &w, int r, bool star, int steps, cudaStream_t s);
 
+// One direct step of a 3-D grid, radius 1 (ffs_march3.cu).
+struct March3Work {
+    const double *in;
+    double *out;
+    double w[27];
+    int n[3], periodic;
+    int slo[3], shi[3];         // cells that are stepped (fixed boundary); the others keep their value
+    int small, tiles[2], chunk, units; // set by march3_units
+};
+cudaError_t prepare_march3();
+double march3_units(March3Work *w, int taps, int num_sms); // the modelled seconds
+cudaError_t launch_march3d(const March3Work &w, bool star, cudaStream_t s);
+
+// `steps` direct steps of a 1-D grid, radius 1 .. 4 (ffs_line.cu), k = 8 or 16 cells per lane.
+struct LineWork {
+    const double *in;
+    double *out;
+    double w[9];
+    int64_t n, units; // units: set by launch_line
+    int64_t slo, shi; // cells that are stepped (fixed boundary); the others keep their value
+    int steps, periodic;
+};
+int line_max_steps(int r, int k);
+cudaError_t launch_line(LineWork w, int r, int k, cudaStream_t s);
+
 // Autotuner utilities: a seeded uniform [0, 1) fill, and out[0] = max |y - r|,
 // out[1] = max |r| as ordered bit patterns (out zeroed by the caller).
 cudaError_t launch_fill_uniform(double *d, size_t n, uint64_t seed, cudaStream_t s);

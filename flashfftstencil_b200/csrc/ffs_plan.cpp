@@ -159,13 +159,15 @@ void geometry(const PlanSpec &sp, int tau, PassSpec *ps)
 // Fixed-boundary band: every cell outside the exact window, partitioned into
 // slabs (cell goes to the highest dim in which it is in the band) and boxes
 // small enough that box + r*tau halo fits the band kernel's shared memory.
-void band_boxes(const PlanSpec &sp, PassSpec *ps)
+struct BandSlab {
+    int64_t lo[3], hi[3], chunk[3];
+};
+std::vector<BandSlab> band_slabs(const PlanSpec &sp, const PassSpec &ps)
 {
-    ps->boxes.clear();
-    ps->band_max_vol = 0;
-    if (sp.boundary != FFS_BOUNDARY_FIXED || ps->tau == 0)
-        return;
-    const int64_t rt = (int64_t)sp.radius * ps->tau;
+    std::vector<BandSlab> slabs;
+    if (sp.boundary != FFS_BOUNDARY_FIXED || ps.tau == 0)
+        return slabs;
+    const int64_t rt = (int64_t)sp.radius * ps.tau;
     const size_t tap_bytes = sp.taps.size() * (sizeof(int4) + sizeof(double)) + 64;
     const int64_t vol_limit = (int64_t)((kBandSmemLimit - tap_bytes) / (2 * sizeof(double)));
     for (int d = sp.dim - 1; d >= 0; --d) {
@@ -176,16 +178,16 @@ void band_boxes(const PlanSpec &sp, PassSpec *ps)
                     lo[e] = 0;
                     hi[e] = 1;
                 } else if (e > d) {
-                    lo[e] = ps->vlo[e];
-                    hi[e] = ps->vhi[e];
+                    lo[e] = ps.vlo[e];
+                    hi[e] = ps.vhi[e];
                 } else if (e < d) {
                     lo[e] = 0;
                     hi[e] = sp.n[e];
                 } else if (side == 0) {
                     lo[e] = 0;
-                    hi[e] = ps->vlo[e];
+                    hi[e] = ps.vlo[e];
                 } else {
-                    lo[e] = ps->vhi[e];
+                    lo[e] = ps.vhi[e];
                     hi[e] = sp.n[e];
                 }
             }
@@ -225,26 +227,56 @@ void band_boxes(const PlanSpec &sp, PassSpec *ps)
                     break;
                 chunk[big] = (chunk[big] + 1) / 2;
             }
-            for (int64_t z = lo[2]; z < hi[2]; z += chunk[2])
-                for (int64_t y = lo[1]; y < hi[1]; y += chunk[1])
-                    for (int64_t x = lo[0]; x < hi[0]; x += chunk[0]) {
-                        BandBox b;
-                        const int64_t o[3] = {x, y, z};
-                        int64_t vol = 1;
-                        for (int e = 0; e < 3; ++e) {
-                            b.lo[e] = o[e];
-                            b.ext[e] = (int32_t)std::min<int64_t>(chunk[e], hi[e] - o[e]);
-                            if (e < sp.dim) {
-                                const int64_t L = std::max<int64_t>(o[e] - rt, 0);
-                                const int64_t R = std::min<int64_t>(o[e] + b.ext[e] + rt, sp.n[e]);
-                                vol *= R - L;
-                            }
-                        }
-                        ps->band_max_vol = std::max(ps->band_max_vol, vol);
-                        ps->boxes.push_back(b);
-                    }
+            BandSlab b;
+            for (int e = 0; e < 3; ++e) {
+                b.lo[e] = lo[e];
+                b.hi[e] = hi[e];
+                b.chunk[e] = chunk[e];
+            }
+            slabs.push_back(b);
         }
     }
+    return slabs;
+}
+
+// Largest staged region of the band's boxes: per slab the product of each axis' longest staged run
+// (the boxes are all combinations of the axes' segments).
+int64_t band_max_volume(const PlanSpec &sp, const PassSpec &ps, const std::vector<BandSlab> &slabs)
+{
+    const int64_t rt = (int64_t)sp.radius * ps.tau;
+    int64_t most = 0;
+    for (const BandSlab &b : slabs) {
+        int64_t vol = 1;
+        for (int e = 0; e < sp.dim; ++e) {
+            int64_t run = 0;
+            for (int64_t o = b.lo[e]; o < b.hi[e]; o += b.chunk[e]) {
+                const int64_t end = std::min(o + b.chunk[e], b.hi[e]);
+                run = std::max(run, std::min<int64_t>(end + rt, sp.n[e]) - std::max<int64_t>(o - rt, 0));
+            }
+            vol *= run;
+        }
+        most = std::max(most, vol);
+    }
+    return most;
+}
+
+void band_boxes(const PlanSpec &sp, PassSpec *ps)
+{
+    ps->boxes.clear();
+    const std::vector<BandSlab> slabs = band_slabs(sp, *ps);
+    ps->band_max_vol = band_max_volume(sp, *ps, slabs);
+    for (const BandSlab &b : slabs)
+        for (int64_t z = b.lo[2]; z < b.hi[2]; z += b.chunk[2])
+            for (int64_t y = b.lo[1]; y < b.hi[1]; y += b.chunk[1])
+                for (int64_t x = b.lo[0]; x < b.hi[0]; x += b.chunk[0]) {
+                    BandBox box;
+                    const int64_t o[3] = {x, y, z};
+                    for (int e = 0; e < 3; ++e) {
+                        box.lo[e] = o[e];
+                        box.ext[e] = (int32_t)std::min<int64_t>(b.chunk[e], b.hi[e] - o[e]);
+                    }
+                    ps->boxes.push_back(box);
+                }
 }
 
 // One 32^3 complex tile pair on a four-SM cluster (FP64 butterflies), measured: 27-33 us
@@ -259,19 +291,33 @@ constexpr double kTile32ClustersPerSm = 33.0 / 148.0;
 constexpr double kTile128Seconds = 20e-6;
 
 // Modelled seconds of a pass's band.  Boxes run concurrently, several per SM; a box costs its
-// direct stepping work plus a per-step barrier latency.
+// direct stepping work plus a per-step barrier latency.  Along an axis a slab's boxes have at most
+// two extents (the chunk and a remainder), so the sum needs no list of boxes: a 512^3 shell at
+// large tau has millions, and the models of all step counts took seconds.
 double band_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
 {
     double box_max = 0.0, box_sum = 0.0;
-    for (const BandBox &b : ps.boxes) {
-        double v = 1.0;
-        for (int e = 0; e < sp.dim; ++e)
-            v *= std::min<double>(b.ext[e] + 2.0 * sp.radius * ps.tau, (double)sp.n[e]);
-        const double bt = v * ps.tau * (double)sp.taps.size() / 60e9 + ps.tau * 0.3e-6;
-        box_max = std::max(box_max, bt);
-        box_sum += bt;
+    for (const BandSlab &b : band_slabs(sp, ps)) {
+        double count[3][2] = {{1, 0}, {1, 0}, {1, 0}}, size[3][2] = {{1, 1}, {1, 1}, {1, 1}};
+        for (int e = 0; e < sp.dim; ++e) {
+            const int64_t len = b.hi[e] - b.lo[e], rem = len % b.chunk[e];
+            count[e][0] = (double)(len / b.chunk[e]);
+            count[e][1] = rem ? 1.0 : 0.0;
+            size[e][0] = std::min<double>((double)b.chunk[e] + 2.0 * sp.radius * ps.tau, (double)sp.n[e]);
+            size[e][1] = std::min<double>((double)rem + 2.0 * sp.radius * ps.tau, (double)sp.n[e]);
+        }
+        for (int k = 0; k < 8; ++k) {
+            const int i = k & 1, j = k >> 1 & 1, l = k >> 2;
+            const double boxes = count[0][i] * count[1][j] * count[2][l];
+            if (boxes == 0.0)
+                continue;
+            const double v = size[0][i] * size[1][j] * size[2][l];
+            const double bt = v * ps.tau * (double)sp.taps.size() / 60e9 + ps.tau * 0.3e-6;
+            box_max = std::max(box_max, bt);
+            box_sum += boxes * bt;
+        }
     }
-    return ps.boxes.empty() ? 0.0 : std::max(box_max, box_sum / (num_sms * 4.0)) + 3e-6;
+    return box_sum == 0.0 ? 0.0 : std::max(box_max, box_sum / (num_sms * 4.0)) + 3e-6;
 }
 
 // Model of one pass in seconds (used to pick tau).  Rough per-form constants;
@@ -293,10 +339,6 @@ double pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
         tile_pair_s = kTile32PairSeconds;
     if (sp.dim == 2 && sp.tile == 128)
         tile_pair_s = kTile128Seconds;
-    // an odd row length rules TMA out: the 64 x 64 tiles of a 1999 x 2047 grid took 1.95 times as
-    // long with wrapped plain loads, 1.3 times with clipped ones
-    else if (sp.dim == 2 && sp.form == FFS_FORM_FP64_FFT && (sp.n[0] & 1))
-        tile_pair_s *= sp.boundary == FFS_BOUNDARY_PERIODIC ? 1.9 : 1.3;
     const double waves = std::ceil((double)ps.nitems / (cluster ? std::floor(kTile32ClustersPerSm * num_sms) : num_sms));
     return waves * tile_pair_s + band_cost(sp, ps, num_sms) + 4e-6;
 }
@@ -319,7 +361,6 @@ double model_cost(const PlanSpec &sp, int tau)
 {
     PassSpec ps;
     geometry(sp, tau, &ps);
-    band_boxes(sp, &ps);
     const int passes = (sp.T + tau - 1) / tau;
     return passes * pass_cost(sp, ps, 148);
 }
@@ -346,7 +387,6 @@ void pick_tau(PlanSpec *sp, int tau_override)
         for (int tau = 1; tau <= tau_max; ++tau) {
             PassSpec ps;
             geometry(*sp, tau, &ps);
-            band_boxes(*sp, &ps);
             const int passes = (sp->T + tau - 1) / tau;
             const double c = passes * pass_cost(*sp, ps, 148);
             if (c < best_cost * (1 - 1e-9)) {
@@ -392,6 +432,9 @@ int pick_tile(const PlanSpec &sp, int tau_override)
 constexpr double kMarchFmaPerSecond = 9e12;
 constexpr double kMarchLaunchSeconds = 5e-6; // launch, first rows
 constexpr double kMarchBytesPerSecond = 5e12;
+// 1-D: launch and copies; a step of a warp alone; multiply-adds with every SM busy
+constexpr double kLineLaunchSeconds = 6e-6, kLineStepSeconds = 0.04e-6, kLineCellSeconds = 1.5e-9;
+constexpr double kLineFmaPerSecond = 9e12;
 constexpr double kMarchRowSeconds = 0.13e-6; // a warp alone: one level of one row
 
 // Modelled seconds of `tau` fused steps of one nx x ny region.
@@ -427,14 +470,99 @@ std::string direct_override()
     return env ? env : "";
 }
 
+// Modelled seconds of one direct step of a 3-D grid.
+double march3_cost(const PlanSpec &sp)
+{
+    March3Work w{};
+    for (int d = 0; d < 3; ++d)
+        w.n[d] = (int)sp.n[d];
+    w.periodic = sp.boundary == FFS_BOUNDARY_PERIODIC;
+    return std::max(march3_units(&w, (int)sp.taps.size(), 148), 16.0 * (double)sp.cells / kMarchBytesPerSecond);
+}
+
+// The modelled solve on the form's one-SM tiles, to compare with the other routes.  Corrections to the
+// model that ranks the tiles' own step counts:
+// - 3-D: it counts 3 us per pair of 16^3 tiles (its band and launch terms were fitted with that), but a
+//   pair takes 6 us: 100 x 90 x 70, periodic, T = 10 81 us, 256^3 at T = 4 443 us;
+// - 2-D: an odd row length rules TMA out, and the 64 x 64 tiles of a 1999 x 2047 grid took 1.9 times as
+//   long with wrapped plain loads, 1.3 times with clipped ones;
+// - 1-D: a wave takes 10.5 us, not 6 (16.7 M cells 150 us, 44.3 M 404 us, a few thousand 14.8), and a band
+//   whose boxes fit a warp (256 staged cells) hides beside it (2^20, fixed, T = 64: 14.9 us).
+double tile_route_cost(const PlanSpec &sp)
+{
+    double c = model_cost(sp, sp.tau), more = 0.0;
+    if (sp.form != FFS_FORM_FP64_FFT)
+        return c;
+    if (sp.dim == 3 && sp.tile == 16)
+        more = 3e-6;
+    else if (sp.dim == 2 && sp.tile == 64 && (sp.n[0] & 1))
+        more = 5.7e-6 * (sp.boundary == FFS_BOUNDARY_PERIODIC ? 0.9 : 0.3);
+    else if (sp.dim == 1)
+        more = 4.5e-6;
+    PassSpec ps;
+    geometry(sp, sp.tau, &ps);
+    c += sp.passes * std::ceil((double)ps.nitems / 148) * more;
+    if (sp.dim == 1 && ps.nitems > 0 && 3 * sp.radius * sp.tau <= 256)
+        c -= sp.passes * band_cost(sp, ps, 148);
+    return c;
+}
+
+double pick_direct3(PlanSpec *sp, bool forced)
+{
+    if (sp->radius != 1 || sp->n[0] >= 1 << 30 || sp->n[2] >= 1 << 30 || sp->n[0] * sp->n[1] >= 1ll << 31)
+        return INFINITY;
+    sp->tau = sp->tau_last = 1;
+    sp->passes = sp->T;
+    return forced ? 0.0 : sp->T * march3_cost(*sp);
+}
+
+// Modelled seconds of `steps` direct steps of a line, k cells per lane.
+double line_cost(const PlanSpec &sp, int k, int steps)
+{
+    const double taps = 2.0 * sp.radius + 1, n = (double)sp.n[0];
+    const double units = std::ceil(n / (32.0 * k - 2.0 * sp.radius * steps));
+    // a warp loads, steps and stores in turn, so bytes and multiply-adds add up (fewer warps per SM
+    // with 16 cells a lane)
+    return std::max(16.0 * n / (k == 8 ? 5e12 : 4e12) + units * 32 * k * steps * taps / kLineFmaPerSecond,
+                    steps * (kLineStepSeconds + kLineCellSeconds * taps * k)) +
+           kLineLaunchSeconds;
+}
+
+double pick_direct1(PlanSpec *sp, bool forced)
+{
+    double best = INFINITY;
+    for (int k : {8, 16}) {
+        const int most = line_max_steps(sp->radius, k);
+        if (most == 0)
+            continue;
+        const int least = (sp->T + most - 1) / most;
+        for (int passes = least; passes <= std::min(sp->T, 3 * least); ++passes) {
+            const int tau = (sp->T + passes - 1) / passes;
+            const double c = passes * line_cost(*sp, k, tau);
+            if (c < best) {
+                best = c;
+                sp->line_k = k;
+                sp->tau = tau;
+                sp->passes = (sp->T + tau - 1) / tau;
+                sp->tau_last = sp->T - (sp->passes - 1) * tau;
+            }
+        }
+    }
+    return forced && best < INFINITY ? 0.0 : best;
+}
+
 // The whole solve stepped directly: fills tau, passes and the kernel, returns seconds.
 double pick_direct(PlanSpec *sp)
 {
     const int r = sp->radius;
+    const std::string only = direct_override();
+    if (sp->dim == 1)
+        return only == "blocks" ? INFINITY : pick_direct1(sp, only == "march");
+    if (sp->dim == 3)
+        return only == "blocks" ? INFINITY : pick_direct3(sp, only == "march");
     if (sp->dim != 2 || march_max_tau(r, sp->star) == 0 || sp->n[0] >= 1 << 30 || sp->n[1] >= 1 << 30)
         return INFINITY;
     double best = INFINITY;
-    const std::string only = direct_override();
     for (bool blocks : {false, true}) {
         if (only == (blocks ? "march" : "blocks"))
             continue;
@@ -460,6 +588,10 @@ double pick_direct(PlanSpec *sp)
 // Modelled seconds of one direct pass.
 double direct_cost(const PlanSpec &sp, int tau)
 {
+    if (sp.dim == 1)
+        return line_cost(sp, sp.line_k, tau);
+    if (sp.dim == 3)
+        return march3_cost(sp);
     const double U = step_width(sp.radius, tau);
     return sp.blocks ? step_cost(sp, std::ceil(sp.n[0] / U) * std::ceil(sp.n[1] / U), tau)
                      : march_cost(sp, (double)sp.n[0], (double)sp.n[1], tau);
@@ -584,7 +716,7 @@ double pick_wide(PlanSpec *sp)
         t.tile = 2048;
         geometry(t, tau, &ps);
         if (!t.frame)
-            band_boxes(t, &ps);
+            ps.band_max_vol = band_max_volume(t, ps, band_slabs(t, ps));
         if (ps.band_max_vol > 0 && band_smem_bytes(ps.band_max_vol, (int)t.taps.size()) > kBandSmemLimit)
             continue;
         for (int ex : kWideEdges)
@@ -1216,9 +1348,9 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
                         sp.taps.push_back(make_int4(dx, dy, dz, idx));
                 }
     }
-    sp.star = sp.dim == 2;
+    sp.star = true;
     for (const int4 &t : sp.taps)
-        sp.star &= t.x == 0 || t.y == 0;
+        sp.star &= (t.x != 0) + (t.y != 0) + (t.z != 0) <= 1;
     if (sp.form == FFS_FORM_OZAKI_I8 && sp.slices == 0) { // a calibrated count for this class wins
         const int tuned = tune_lookup(slice_key(sp));
         sp.slices = (tuned >= 4 && tuned <= 8) ? tuned : kDefaultOzakiSlices;
@@ -1241,11 +1373,13 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
     pick_tau(&sp, p.tau);
     // wide tiles and direct stepping: only where the caller left both the edge and the step count
     // open; a measured choice for the class wins over the model, as for the edges
-    if (edge_open && p.tau == 0) {
-        const int measured = route == kRouteAuto ? tune_lookup(tile_key(sp)) : 0;
-        const bool edge_measured = measured > kDirectTuned; // 64, 128 (2D), 16, 32 (3D)
+    if (p.tile == 0 && p.tau == 0 && sp.T > 0 && sp.form == FFS_FORM_FP64_FFT) {
+        int measured = route == kRouteAuto ? tune_lookup(tile_key(sp)) : 0;
+        if (sp.dim == 1 && measured == 0 && route == kRouteAuto && tune_lookup(tune_key(sp)) > 0)
+            measured = sp.tile; // a table written before 1-D had two routes
+        const bool edge_measured = measured > kDirectTuned; // 4096 (1D), 64, 128 (2D), 16, 32 (3D)
         double best = route >= kRouteWide || measured == kWideTuned || measured == kDirectTuned ? INFINITY
-                                                                                              : model_cost(sp, sp.tau);
+                                                                                              : tile_route_cost(sp);
         if (edge_measured)
             best = 0.0;
         PlanSpec w = sp, d = sp;
@@ -1266,7 +1400,7 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
                 best = c;
                 sp = std::move(d);
                 sp.direct = true;
-                sp.tile = 128;
+                sp.tile = sp.dim == 1 ? 32 * sp.line_k : sp.dim == 2 ? 128 : 64;
             }
         }
     }

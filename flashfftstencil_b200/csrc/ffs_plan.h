@@ -56,7 +56,8 @@ struct PlanSpec {
     int wtile[3] = {1, 1, 1};    // wide tile edges
     int wchunk = 0;              // tiles per chunk of a wide pass (one workspace)
     bool direct = false;         // stepped directly, tau steps per pass, no transform:
-    bool blocks = false;         // by blocks (ffs_step.cu), else by marching warps (ffs_march.cu)
+    bool blocks = false;         // 2-D: by blocks (ffs_step.cu), else by marching warps (ffs_march.cu)
+    int line_k = 0;              // 1-D: cells per lane (ffs_line.cu)
     bool frame = false;          // the wide tiles' band is stepped by ffs_step.cu (no band boxes)
     bool star = false;           // 2-D: all taps on the axes
     int tau = 0, tau_last = 0, passes = 0;

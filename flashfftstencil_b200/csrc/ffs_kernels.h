@@ -149,7 +149,7 @@ struct MarchRegion {
     int ox0, ox1, oy0, oy1; // cells to write
     int strips, chunk, first_unit; // set by march_units
 };
-constexpr int kMarchRegions = 12;
+constexpr int kMarchRegions = 4;
 struct MarchWork {
     MarchRegion reg[kMarchRegions];
     double w[25]; // dense (2r+1)^2 taps

@@ -14,6 +14,7 @@
 // short lines.  K = 8 has twice the warps, K = 16 half the margin: long runs take 16.
 #include <type_traits>
 
+#include "ffs_chain.cuh"
 #include "ffs_kernels.h"
 
 namespace ffst {
@@ -26,6 +27,7 @@ __global__ void __launch_bounds__(32 * kWarps) line_kernel(const __grid_constant
 {
     constexpr int W = 32 * K, PITCH = W + 32;
     __shared__ double stage[kWarps][PITCH];
+    chain_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t u = (int64_t)blockIdx.x * kWarps + warp;
     if (u >= p.units)
@@ -106,11 +108,8 @@ template <int R>
 cudaError_t launch(const LineWork &w, int k, cudaStream_t s)
 {
     const unsigned blocks = (unsigned)((w.units + kWarps - 1) / kWarps);
-    if (k == 8)
-        line_kernel<R, 8><<<blocks, 32 * kWarps, 0, s>>>(w);
-    else
-        line_kernel<R, 16><<<blocks, 32 * kWarps, 0, s>>>(w);
-    return cudaGetLastError();
+    return k == 8 ? launch_chained(line_kernel<R, 8>, blocks, 32 * kWarps, 0, s, w)
+                  : launch_chained(line_kernel<R, 16>, blocks, 32 * kWarps, 0, s, w);
 }
 
 } // namespace line

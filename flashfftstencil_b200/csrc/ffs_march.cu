@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "ffs_chain.cuh"
 #include "ffs_kernels.h"
 
 namespace ffst {
@@ -62,6 +63,7 @@ template <int R, bool STAR, bool FIXED, int TAU>
 __global__ void __launch_bounds__(32 * kWarps, blocks_per_sm(R, STAR, FIXED, TAU)) march2d_kernel(const __grid_constant__ MarchWork p)
 {
     extern __shared__ __align__(16) double stage[];
+    chain_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int u = blockIdx.x * kWarps + warp;
     if (u >= p.units)
@@ -251,11 +253,8 @@ template <int R, bool STAR, int TAU>
 cudaError_t launch(const MarchWork &w, cudaStream_t s)
 {
     const int blocks = (w.units + kWarps - 1) / kWarps;
-    if (w.periodic)
-        march2d_kernel<R, STAR, false, TAU><<<blocks, 32 * kWarps, kSmemBytes, s>>>(w);
-    else
-        march2d_kernel<R, STAR, true, TAU><<<blocks, 32 * kWarps, kSmemBytes, s>>>(w);
-    return cudaGetLastError();
+    return w.periodic ? launch_chained(march2d_kernel<R, STAR, false, TAU>, blocks, 32 * kWarps, kSmemBytes, s, w)
+                      : launch_chained(march2d_kernel<R, STAR, true, TAU>, blocks, 32 * kWarps, kSmemBytes, s, w);
 }
 
 // Most steps of one launch: 2 r K accumulators per level beside the taps.

@@ -19,6 +19,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "ffs_chain.cuh"
 #include "ffs_kernels.h"
 
 namespace ffst {
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(NT, 2) march3d_kernel(const __grid_constant__ 
 {
     constexpr int TX = T::TX, TY = T::TY, kRows = T::kRows, PX = T::PX, PY = T::PY, kPlane = T::kPlane;
     extern __shared__ __align__(16) double smem[];
+    chain_wait();
     int u = blockIdx.x;
     const int chunk = u / (p.tiles[0] * p.tiles[1]);
     u -= chunk * p.tiles[0] * p.tiles[1];
@@ -223,8 +225,7 @@ cudaError_t launch(const March3Work &w, cudaStream_t s)
     if (w.units <= 0) // set-up call
         return cudaFuncSetAttribute(march3d_kernel<T, STAR, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)T::kSmemBytes);
-    march3d_kernel<T, STAR, FIXED><<<w.units, NT, T::kSmemBytes, s>>>(w);
-    return cudaGetLastError();
+    return launch_chained(march3d_kernel<T, STAR, FIXED>, (unsigned)w.units, NT, T::kSmemBytes, s, w);
 }
 
 template <class T>
@@ -240,11 +241,13 @@ cudaError_t dispatch(const March3Work &w, bool star, cudaStream_t s)
     return w.small ? by_boundary<Small>(w, star, s) : by_boundary<Large>(w, star, s);
 }
 
-// A plane of an SM's two blocks (half as long with one block per SM), and per tap.  Measured, us a step,
+// A plane of an SM's two blocks, and per tap (one block per SM takes about half: Heat-3D 100 x 90 x 70 in
+// 144 units of 6 planes 5.8 us a step, in 288 of 3 planes 7.8; but Box3D27P 512^3 in 128 units 667, in 1152
+// 453).  Measured, us a step,
 // Large / Small: Heat-3D 65 x 33 x 9 4.8 / 3.4, 100 x 90 x 70 6.2 / 5.8, 236 x 144 x 99 15.0 / 15.6, 256^3 57 / 60;
 // Box3D27P 100 x 90 x 70 7.5 / 7.1, 256^3 60 / 64; Large at 512^3, fixed, 413 and 453.
 constexpr double kMarch3PlaneSeconds = 1.5e-6, kMarch3TapSeconds = 0.012e-6;
-constexpr double kMarch3SmallPlaneSeconds = 0.68e-6, kMarch3SmallTapSeconds = 0.007e-6;
+constexpr double kMarch3SmallPlaneSeconds = 0.85e-6, kMarch3SmallTapSeconds = 0.007e-6;
 constexpr double kMarch3LaunchSeconds = 2e-6;
 
 } // namespace march3
@@ -273,15 +276,17 @@ double march3_units(March3Work *w, int taps, int num_sms)
         const int tx = small ? march3::Small::TX : march3::Large::TX, ty = small ? march3::Small::TY : march3::Large::TY;
         const int x = (in.n[0] + tx - 1) / tx, y = (in.n[1] + ty - 1) / ty;
         using namespace march3;
-        const double plane = (small ? kMarch3SmallPlaneSeconds + kMarch3SmallTapSeconds * taps
-                                    : kMarch3PlaneSeconds + kMarch3TapSeconds * taps) *
-                             (in.periodic ? 1.0 : 1.15);
+        // a plane of an SM's two blocks, and of one block alone
+        const double fixed = in.periodic ? 1.0 : 1.15, base = small ? kMarch3SmallPlaneSeconds : kMarch3PlaneSeconds,
+                     tap = (small ? kMarch3SmallTapSeconds : kMarch3TapSeconds) * taps;
+        const double two = fixed * (base + tap),
+                     one = (in.periodic ? 0.8 : 1.1) * (0.5 * base + 1.2 * tap);
         for (int n = 1; n <= in.n[2] && n <= 4096; ++n) {
             const int len = (in.n[2] + n - 1) / n;
             if ((in.n[2] + len - 1) / len != n)
                 continue;
             const int64_t units = (int64_t)x * y * n;
-            const double cost = std::ceil((double)units / (2.0 * num_sms)) * (len + 4) * plane * (units <= num_sms ? 0.5 : 1.0);
+            const double cost = std::ceil((double)units / (2.0 * num_sms)) * (len + 4) * (units <= num_sms ? one : two);
             if (units < INT32_MAX && cost < best) {
                 best = cost;
                 w->small = small;

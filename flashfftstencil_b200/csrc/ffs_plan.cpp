@@ -523,9 +523,8 @@ double line_cost(const PlanSpec &sp, int k, int steps)
     const double units = std::ceil(n / (32.0 * k - 2.0 * sp.radius * steps));
     // a warp loads, steps and stores in turn, so bytes and multiply-adds add up (fewer warps per SM
     // with 16 cells a lane)
-    return std::max(16.0 * n / (k == 8 ? 5e12 : 4e12) + units * 32 * k * steps * taps / kLineFmaPerSecond,
-                    steps * (kLineStepSeconds + kLineCellSeconds * taps * k)) +
-           kLineLaunchSeconds;
+    const double busy = 16.0 * n / (k == 8 ? 5e12 : 4e12) + units * 32 * k * steps * taps / kLineFmaPerSecond + 2.5e-6;
+    return std::max(busy, steps * (kLineStepSeconds + kLineCellSeconds * taps * k) + kLineLaunchSeconds);
 }
 
 double pick_direct1(PlanSpec *sp, bool forced)
@@ -1604,10 +1603,15 @@ void fill_plan_info(const PlanSpec &sp, ffs_plan_info *info)
             // both ways, u/2 packed rows back; plus the spectrum product and the packing
             auto line = [](double e) { return e * (std::log2(e) * 176 / 64 + (e > 256 ? 2 : 1) * 90 / 16.0); };
             const double nx = sp.wtile[0], ny = sp.wtile[1];
-            info->flops_per_pass = 2.0 * (nx * nx * ny + nx * ny * ny) * 4.0 * (double)ps.nitems;
-            info->exec_flops_per_pass = ((ny + (double)ps.wuseful[1]) / 2 * line(nx) + (nx + 2) * line(ny) +
-                                         10.0 * (nx / 2 + 1) * ny) *
-                                        (double)ps.nitems;
+            if (sp.dim == 1) { // both ways and the spectrum, per pair
+                info->flops_per_pass = 2.0 * nx * nx * 8.0 * (double)ps.nitems / 2;
+                info->exec_flops_per_pass = (2 * line(nx) + 6.0 * nx) * (double)ps.nitems / 2;
+            } else {
+                info->flops_per_pass = 2.0 * (nx * nx * ny + nx * ny * ny) * 4.0 * (double)ps.nitems;
+                info->exec_flops_per_pass = ((ny + (double)ps.wuseful[1]) / 2 * line(nx) + (nx + 2) * line(ny) +
+                                             10.0 * (nx / 2 + 1) * ny) *
+                                            (double)ps.nitems;
+            }
         } else if (sp.form == FFS_FORM_FP64_FFT && sp.dim == 1) {
             // 256 DFT-64 lines per pair (64 rows, 2 x 64 columns, 64 rows) of 8 x (2 x 56 + 7 x 6),
             // two 4096-point twiddle passes (12 per element: table product and multiply), spectrum

@@ -18,6 +18,7 @@
 // Bound: the FP64 pipe within a step, the barrier and the shuffles' latency between steps.
 #include <algorithm>
 
+#include "ffs_chain.cuh"
 #include "ffs_kernels.h"
 
 namespace ffst {
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) step2d_kernel(const __grid_con
     extern __shared__ __align__(16) double edges[];
     auto edge = reinterpret_cast<double (*)[kWarps][2 * R][W]>(edges); // [step & 1][warp][first, last r rows]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    chain_wait();
     int u = blockIdx.x, k = 0;
     for (int i = 1; i < p.nregions; ++i)
         if (u >= p.reg[i].first_unit)
@@ -190,8 +192,7 @@ cudaError_t launch(const MarchWork &w, int steps, cudaStream_t s)
     constexpr size_t smem = (size_t)2 * kWarps * 2 * R * W * sizeof(double);
     if (w.units <= 0) // set-up call
         return cudaFuncSetAttribute(step2d_kernel<R, STAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    step2d_kernel<R, STAR><<<w.units, 32 * kWarps, smem, s>>>(w, steps);
-    return cudaGetLastError();
+    return launch_chained(step2d_kernel<R, STAR>, (unsigned)w.units, 32 * kWarps, smem, s, w, steps);
 }
 
 cudaError_t dispatch(const MarchWork &w, int r, bool star, int steps, cudaStream_t s)

@@ -19,6 +19,10 @@
 // like the one-SM tiles do.
 #include "ffs_wide.cuh"
 
+#include <algorithm>
+
+#include "ffs_band.cuh"
+#include "ffs_chain.cuh"
 #include "ffs_kernels.h"
 
 namespace ffst {
@@ -65,6 +69,7 @@ __global__ void __launch_bounds__(kRowThreads, row_blocks_per_sm(N)) rows_fwd_ke
 {
     using S = RowShape<N>;
     extern __shared__ __align__(16) double2 smem[];
+    chain_wait();
     const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;
     constexpr int LPB = kRowThreads / S::L;
     const int half = p.tile[1] >> 1;
@@ -122,6 +127,7 @@ __global__ void __launch_bounds__(col_threads(N), col_blocks_per_sm(N)) cols_ker
     using S = ColShape<N>;
     constexpr int C = col_count<N>();
     extern __shared__ __align__(16) double2 smem[];
+    chain_wait();
     const int c = threadIdx.x % C, t = threadIdx.x / C;
     const int hx = p.tile[0] >> 1;
     const int groups = hx / C + 1;
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(kRowThreads, row_blocks_per_sm(N)) rows_inv_ke
 {
     using S = RowShape<N>;
     extern __shared__ __align__(16) double2 smem[];
+    chain_wait();
     const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;
     constexpr int LPB = kRowThreads / S::L;
     const int half = p.tile[1] >> 1;
@@ -326,13 +333,12 @@ cudaError_t rows(const WideWork &w, bool inverse, cudaStream_t s)
     constexpr int LPB = kRowThreads / RowShape<N>::L;
     const size_t smem = sizeof(double2) * RowShape<N>::SLOTS * LPB;
     if (!inverse) {
-        rows_fwd_kernel<N><<<(unsigned)((int64_t)w.ntiles * (w.tile[1] / 2) / LPB), kRowThreads, smem, s>>>(w);
-    } else {
-        const int pairs = ((int)w.useful[1] + 1) / 2;
-        const int64_t blocks = (int64_t)w.ntiles * ((pairs + LPB - 1) / LPB);
-        rows_inv_kernel<N><<<(unsigned)blocks, kRowThreads, smem, s>>>(w);
+        return launch_chained(rows_fwd_kernel<N>, (unsigned)((int64_t)w.ntiles * (w.tile[1] / 2) / LPB), kRowThreads, smem,
+                              s, w);
     }
-    return cudaGetLastError();
+    const int pairs = ((int)w.useful[1] + 1) / 2;
+    const int64_t blocks = (int64_t)w.ntiles * ((pairs + LPB - 1) / LPB);
+    return launch_chained(rows_inv_kernel<N>, (unsigned)blocks, kRowThreads, smem, s, w);
 }
 
 template <int N>
@@ -340,8 +346,7 @@ cudaError_t cols(const WideWork &w, cudaStream_t s)
 {
     constexpr int C = col_count<N>();
     const size_t smem = sizeof(double2) * ColShape<N>::SLOTS * C;
-    cols_kernel<N><<<(unsigned)(w.ntiles * (w.tile[0] / 2 / C + 1)), col_threads(N), smem, s>>>(w);
-    return cudaGetLastError();
+    return launch_chained(cols_kernel<N>, (unsigned)(w.ntiles * (w.tile[0] / 2 / C + 1)), col_threads(N), smem, s, w);
 }
 
 #define FFS_WIDE_BY_EDGE(edge, call)                                                                                \

@@ -465,7 +465,7 @@ static cudaError_t wide_spectra(const ffs_plan *p, double2 *const roots[3])
         w.dim = sp.dim;
         w.r = sp.radius;
         w.tau = sp.pass[k].tau;
-        w.scale = 0.5; // the columns are twice the half spectra
+        w.scale = sp.dim == 1 ? 1.0 : 0.5; // 2-D: the columns are twice the half spectra
         for (int d = 0; d < 3; ++d) {
             w.roots[d] = roots[d];
             w.tile[d] = sp.wtile[d];
@@ -831,7 +831,8 @@ static ffs_status run_pass(const ffs_plan *p, int kind, const double *src, doubl
         const cudaError_t e = direct_pass(p, kind, src, dst, s);
         return e == cudaSuccess ? FFS_OK : fail(FFS_ERR_CUDA, "direct stepping launch: %s", cudaGetErrorString(e));
     }
-    const bool has_band = sp.frame || !ps.boxes.empty();
+    const bool line_tiles = sp.wide && sp.dim == 1; // its launch has the band's boxes as blocks
+    const bool has_band = sp.frame || (!ps.boxes.empty() && !line_tiles);
     const bool fork = ps.nitems > 0 && has_band;
     if (fork) {
         CUDA_TRY(cudaEventRecord(p->ev_fork, s));
@@ -868,7 +869,10 @@ static ffs_status run_pass(const ffs_plan *p, int kind, const double *src, doubl
         const int grid = (int)std::min<int64_t>(ps.nitems, p->num_sms);
         cudaError_t e = cudaSuccess;
         LaunchMark mark(p, s, 0);
-        if (sp.wide) {
+        if (line_tiles) {
+            const BandWork b = band_work(p, kind, src, dst);
+            e = launch_wide1(wide_work(p, kind, src, dst), b, band_smem_bytes(ps.band_max_vol, b.ntaps), s);
+        } else if (sp.wide) {
             e = launch_wide(wide_work(p, kind, src, dst), ps.nitems, sp.wchunk, s);
         } else if (sp.dim == 2 && sp.form == FFS_FORM_FP64_DMMA) {
             CUtensorMap tm;

@@ -95,13 +95,18 @@ __device__ __forceinline__ void process_box(const BandWork &p, int box, unsigned
         const int64_t lo = bx.lo[0] - rt < 0 ? 0 : bx.lo[0] - rt;
         const int64_t hi = bx.lo[0] + bx.ext[0] + rt > p.n[0] ? p.n[0] : bx.lo[0] + bx.ext[0] + rt;
         const int ext = (int)(hi - lo);
-        if (ext <= 32 * kWarpCells && r >= 1 && r <= 4) {
+        if (ext <= 64 * kWarpCells && r >= 1 && r <= 4) { // (8 cells a lane, or 16)
             if (threadIdx.x < 32) {
-                switch (r) {
+                const bool wide = ext > 32 * kWarpCells;
+                switch (wide ? r + 4 : r) {
                 case 1: process_box_1d_warp<1, kWarpCells>(p, bx, lo, ext); break;
                 case 2: process_box_1d_warp<2, kWarpCells>(p, bx, lo, ext); break;
                 case 3: process_box_1d_warp<3, kWarpCells>(p, bx, lo, ext); break;
-                default: process_box_1d_warp<4, kWarpCells>(p, bx, lo, ext); break;
+                case 4: process_box_1d_warp<4, kWarpCells>(p, bx, lo, ext); break;
+                case 5: process_box_1d_warp<1, 2 * kWarpCells>(p, bx, lo, ext); break;
+                case 6: process_box_1d_warp<2, 2 * kWarpCells>(p, bx, lo, ext); break;
+                case 7: process_box_1d_warp<3, 2 * kWarpCells>(p, bx, lo, ext); break;
+                default: process_box_1d_warp<4, 2 * kWarpCells>(p, bx, lo, ext); break;
                 }
             }
             return;

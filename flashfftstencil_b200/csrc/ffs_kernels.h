@@ -137,6 +137,8 @@ struct BandWork {
     int *status;
     int warp_rows;         // 2-D 3 x 3 box: most staged widths are multiples of 32, step by warp rows
 };
+// 1-D wide tiles (pairs of 1024 .. 4096 cells) and the fixed boundary's boxes in one launch.
+cudaError_t launch_wide1(const WideWork &w, const BandWork &band, size_t band_smem, cudaStream_t s);
 cudaError_t prepare_band(size_t max_smem);
 
 // Direct stepping of 2-D regions in registers (ffs_march.cu).  Coordinates are the grid's:

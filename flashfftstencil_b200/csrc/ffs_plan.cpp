@@ -623,6 +623,10 @@ constexpr size_t kWideChunkBytes = (size_t)1 << 30;
 double wide_row_seconds(int n) { return n == 256 ? 5.0e-12 : n == 512 ? 5.2e-12 : n == 1024 ? 5.7e-12 : 5.0e-12; }
 double wide_col_seconds(int n) { return n == 256 ? 4.0e-12 : n == 512 ? 4.8e-12 : n == 1024 ? 5.6e-12 : 7.2e-12; }
 constexpr double kWideLaunchSeconds = 4.5e-6;
+// 1-D: 148 SMs of 8192 points, a few lines alone, and the launch (44.3 M cells 228 us, 10000 10.6)
+constexpr double kWide1WaveSeconds = 12e-6, kWide1LeastSeconds = 7.6e-6, kWide1LaunchSeconds = 3e-6;
+
+double wide1_pass_cost(const PlanSpec &sp, const PassSpec &ps);
 
 // FFS_WIDE_TILE: "0" keeps wide tiles off, "512x1024" takes that edge wherever it fits.
 // Returns -1 off, 0 the model's choice, 1 forced.
@@ -638,7 +642,8 @@ int wide_override(int dim, int tile[3])
     if (got != dim)
         return 0;
     for (int d = 0; d < dim; ++d) {
-        if (std::find(std::begin(kWideEdges), std::end(kWideEdges), v[d]) == std::end(kWideEdges))
+        if (dim == 1 ? v[d] != 1024 && v[d] != 2048 && v[d] != 4096
+                     : std::find(std::begin(kWideEdges), std::end(kWideEdges), v[d]) == std::end(kWideEdges))
             return 0;
         tile[d] = v[d];
     }
@@ -658,7 +663,7 @@ bool wide_geometry(const PlanSpec &sp, PassSpec *ps)
             continue;
         const int h = sp.radius * ps->tau;
         const int64_t u = sp.wtile[d] - 2 * h, w = ps->vhi[d] - ps->vlo[d];
-        if (u < 16 || sp.n[d] < 128) // 128: rows_fwd steps up to 128 cells around a periodic axis at once
+        if (u < 16 || (sp.dim > 1 && sp.n[d] < 128)) // rows_fwd steps up to 128 cells around a periodic axis at once
             return false;
         if (w <= 0) { // no exact window: the band takes the whole grid
             ps->nitems = 0;
@@ -675,12 +680,16 @@ bool wide_geometry(const PlanSpec &sp, PassSpec *ps)
 
 int wide_chunk(const PlanSpec &sp, int64_t tiles)
 {
+    if (sp.dim == 1) // (no workspace)
+        return 0;
     const int64_t c = (int64_t)(kWideChunkBytes / wide_tile_bytes(sp.wtile));
     return (int)std::max<int64_t>(1, std::min(c, tiles));
 }
 
 double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
 {
+    if (sp.dim == 1)
+        return wide1_pass_cost(sp, ps);
     const double pts = (double)sp.wtile[0] * sp.wtile[1] * sp.wtile[2] * (double)ps.nitems;
     const double chunks = std::ceil((double)ps.nitems / wide_chunk(sp, ps.nitems));
     const double tiles = pts * (wide_row_seconds(sp.wtile[0]) + wide_col_seconds(sp.wtile[1])) +
@@ -692,6 +701,50 @@ double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
     return std::max(tiles + 0.7 * busy, band);
 }
 
+// 1-D: seconds of one pass.  An SM holds 8192 complex points (16384 tile cells) at a time.
+double wide1_pass_cost(const PlanSpec &sp, const PassSpec &ps)
+{
+    const double waves = (double)ps.nitems * sp.wtile[0] / (148.0 * 16384);
+    double band = 0.0; // a box steps by one warp up to 512 staged cells, else by a block with a barrier per step
+    if (sp.boundary == FFS_BOUNDARY_FIXED)
+        band = ps.tau * (2.0 * sp.radius * ps.tau <= 512 ? 0.01e-6 + 0.06e-6 * sp.radius : 0.5e-6);
+    // 2^20 cells at T = 64 10.6 us with 2048 (12.8 with 1024, 11.2 with 4096), 16.7 M at T = 32 87 (90, 92)
+    const double edge = sp.wtile[0] == 1024 ? 1.08 : sp.wtile[0] == 4096 ? 1.04 : 1.0;
+    return std::max(edge * std::max(waves * kWide1WaveSeconds, kWide1LeastSeconds), band + 3e-6) + kWide1LaunchSeconds;
+}
+
+double pick_wide1(PlanSpec *sp, int forced)
+{
+    double best = INFINITY;
+    PlanSpec t = *sp;
+    t.wide = true;
+    for (int passes = 1; passes <= std::min(sp->T, 8); ++passes) {
+        const int tau = (sp->T + passes - 1) / passes;
+        if ((sp->T + tau - 1) / tau != passes)
+            continue;
+        for (int edge : {1024, 2048, 4096}) {
+            // (a tile wraps around a periodic line at most once)
+            if ((forced && edge != forced) || edge > sp->n[0] || 2 * round_even(sp->radius * tau) + 16 > edge)
+                continue;
+            PassSpec ps;
+            t.tile = t.wtile[0] = edge;
+            geometry(t, tau, &ps);
+            if (band_smem_bytes(band_max_volume(t, ps, band_slabs(t, ps)), (int)t.taps.size()) > kBandSmemLimit ||
+                !wide_geometry(t, &ps) || ps.nitems == 0)
+                continue;
+            const double c = passes * wide1_pass_cost(t, ps);
+            if (c < best) {
+                best = c;
+                sp->wtile[0] = edge;
+                sp->tau = tau;
+                sp->passes = passes;
+                sp->tau_last = sp->T - (passes - 1) * tau;
+            }
+        }
+    }
+    return forced && best < INFINITY ? 0.0 : best;
+}
+
 // Fills the wide tile, tau and passes of `sp` with the cheapest modelled choice; returns its
 // seconds (infinite when no wide tile fits).
 double pick_wide(PlanSpec *sp)
@@ -699,8 +752,10 @@ double pick_wide(PlanSpec *sp)
     double best = INFINITY;
     int forced[3] = {0, 0, 1};
     const int mode = wide_override(sp->dim, forced);
-    if (sp->form != FFS_FORM_FP64_FFT || sp->dim != 2 || sp->T == 0 || mode < 0)
+    if (sp->form != FFS_FORM_FP64_FFT || sp->dim > 2 || sp->T == 0 || mode < 0)
         return best;
+    if (sp->dim == 1)
+        return pick_wide1(sp, mode > 0 ? forced[0] : 0);
     PlanSpec t = *sp;
     t.wide = true;
     t.frame = sp->frame = sp->boundary == FFS_BOUNDARY_FIXED && march_max_tau(sp->radius, sp->star) > 0 && sp->n[0] < 1 << 30 &&

@@ -228,6 +228,99 @@ __global__ void __launch_bounds__(kRowThreads, row_blocks_per_sm(N)) rows_inv_ke
     }
 }
 
+// ---- 1-D: a pair of tiles per line ----
+//
+// Two tiles of N cells are one complex line (re = tile 2q, im = tile 2q + 1) that stays in its
+// threads' registers: forward, spectrum, inverse, cropped stores, four exchanges and no other
+// shared-memory traffic.  The one-SM tile (ffs_fft1d.cu) stages 4096-cell pairs through shared
+// memory, one per SM, 10.5 us a wave; here an SM holds 8192 points in lines of 1024 to 4096, so short
+// grids spread over more SMs.  The fixed boundary's boxes are blocks of the same launch.
+
+constexpr int kLineThreads = 256;
+template <int N>
+using LineShape = Shape<N, 16>;
+
+// (not inlined: inside the kernel its registers made the lines' code spill)
+__device__ __noinline__ void band_block(const BandWork &band, int box, unsigned char *smem)
+{
+    band::process_box<1>(band, box, smem, kLineThreads);
+}
+
+template <int N>
+__global__ void __launch_bounds__(kLineThreads, 2) line_tiles_kernel(const __grid_constant__ WideWork p,
+                                                                     const __grid_constant__ BandWork band, int tile_blocks)
+{
+    using S = LineShape<N>;
+    constexpr int LPB = kLineThreads / S::L;
+    extern __shared__ __align__(16) double2 smem[];
+    chain_wait();
+    if ((int)blockIdx.x >= tile_blocks) {
+        band_block(band, (int)blockIdx.x - tile_blocks, reinterpret_cast<unsigned char *>(smem));
+        return;
+    }
+    const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;
+    const int64_t q = (int64_t)blockIdx.x * LPB + l;
+    const bool ona = 2 * q < p.nt[0], onb = 2 * q + 1 < p.nt[0];
+    const int64_t n = p.n[0], oa = p.org[0] + 2 * q * p.useful[0], ob = oa + p.useful[0]; // the tiles' first cells
+    double xr[S::P], xi[S::P];
+    if (oa >= 0 && ob + N <= n && onb) { // both tiles inside the grid
+        const double *a0 = p.in + oa + t, *b0 = p.in + ob + t;
+#pragma unroll
+        for (int a = 0; a < S::P; ++a) {
+            xr[a] = __ldg(a0 + S::L * a);
+            xi[a] = __ldg(b0 + S::L * a);
+        }
+    } else {
+#pragma unroll
+        for (int a = 0; a < S::P; ++a) {
+            int64_t x = oa + t + S::L * a, y = x + p.useful[0];
+            if (p.periodic) { // (N <= n: at most one period off)
+                x += x < 0 ? n : x >= n ? -n : 0;
+                y += y < 0 ? n : y >= n ? -n : 0;
+            }
+            xr[a] = ona && x >= 0 && x < n ? __ldg(p.in + x) : 0.0;
+            xi[a] = onb && y >= 0 && y < n ? __ldg(p.in + y) : 0.0;
+        }
+    }
+    double2 *sm = smem + l * S::SLOTS;
+    line_fft<N, false, 1, S::P>(xr, xi, t, sm, p.tw[0], BlockSync());
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int f = t + S::L * a; // real weights: S(-f) = conj S(f)
+        const double2 s = p.spec[a < S::P / 2 ? f : N - f];
+        f128::cmul(xr[a], xi[a], s.x, a < S::P / 2 ? s.y : -s.y);
+        if (a % 4 == 3)
+            f128::hoist_fence();
+    }
+    __syncthreads(); // the forward transform's last gets before the inverse's first puts
+    int ti = t;
+    asm volatile("" : "+r"(ti)); // hides that the inverse reads the same twiddles: kept over, they spill
+    line_fft<N, true, 1, S::P>(xr, xi, ti, sm, p.tw[0], BlockSync());
+    // useful cells below vhi
+    const int lo = p.halo[0];
+    const int64_t end = lo + p.useful[0];
+    const int ha = ona ? (int)min(end, p.vhi[0] - oa) : 0, hb = onb ? (int)min(end, p.vhi[0] - ob) : 0;
+    double *a1 = p.out + oa + t, *b1 = p.out + ob + t;
+#pragma unroll
+    for (int a = 0; a < S::P; ++a) {
+        const int c = t + S::L * a;
+        if (c >= lo && c < ha)
+            a1[S::L * a] = xr[a];
+        if (c >= lo && c < hb)
+            b1[S::L * a] = xi[a];
+    }
+}
+
+template <int N>
+cudaError_t line_tiles(const WideWork &w, const BandWork &band, size_t band_smem, cudaStream_t s)
+{
+    using S = LineShape<N>;
+    constexpr int LPB = kLineThreads / S::L;
+    const size_t smem = std::max(sizeof(double2) * S::SLOTS * LPB, band_smem);
+    const int64_t blocks = ((w.nt[0] + 1) / 2 + LPB - 1) / LPB;
+    return launch_chained(line_tiles_kernel<N>, (unsigned)(blocks + band.nboxes), kLineThreads, smem, s, w, band, (int)blocks);
+}
+
 // ---- the spectrum S^tau, in double-double arithmetic ----
 //
 // S(k)^tau by repeated squaring multiplies the relative error of S by tau, so plain FP64
@@ -367,11 +460,35 @@ cudaError_t cols_any(const WideWork &w, cudaStream_t s)
     FFS_WIDE_BY_EDGE(w.tile[1], (cols<N>(w, s)))
 }
 
+constexpr size_t kLineSmemLimit = 200 * 1024; // (a band box may need more than the lines)
+
+template <int N>
+cudaError_t prepare_line()
+{
+    return cudaFuncSetAttribute(line_tiles_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLineSmemLimit);
+}
+
 } // namespace wide
+
+cudaError_t launch_wide1(const WideWork &w, const BandWork &band, size_t band_smem, cudaStream_t s)
+{
+    switch (w.tile[0]) {
+    case 1024: return wide::line_tiles<1024>(w, band, band_smem, s);
+    case 2048: return wide::line_tiles<2048>(w, band, band_smem, s);
+    case 4096: return wide::line_tiles<4096>(w, band, band_smem, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
 
 cudaError_t prepare_wide()
 {
-    cudaError_t e = wide::prepare_one<256>();
+    cudaError_t e = wide::prepare_line<1024>();
+    if (e == cudaSuccess)
+        e = wide::prepare_line<2048>();
+    if (e == cudaSuccess)
+        e = wide::prepare_line<4096>();
+    if (e == cudaSuccess)
+        e = wide::prepare_one<256>();
     if (e == cudaSuccess)
         e = wide::prepare_one<512>();
     if (e == cudaSuccess)

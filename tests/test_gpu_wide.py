@@ -96,3 +96,47 @@ def test_repeats_use_each_input(monkeypatch):
             plan.run(x, o, stream=s)
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(first, outs))
+
+
+def _line(n, T, boundary, radius, in_place=False, offset=0):
+    import torch
+    w = seeded_weights(1, radius, 3)
+    plan = ffs.Plan(1, None, (n,), T, weights=w, radius=radius, boundary=boundary, form="auto")
+    x = seeded_grid((n,), 4)
+    buf = torch.empty(n + offset, dtype=torch.float64, device="cuda")
+    d = buf[offset:]
+    d.copy_(torch.from_numpy(x))
+    out = d if in_place else torch.full_like(d, float("nan"))
+    plan.run(d, out)
+    torch.cuda.synchronize()
+    ref = oracle.run(x, w, radius, T, oracle.FIXED if boundary == "fixed" else oracle.PERIODIC)
+    return plan, rel_errors(out.cpu().numpy(), ref)[0]
+
+
+@pytest.mark.parametrize("boundary", ["fixed", "periodic"])
+@pytest.mark.parametrize("edge", [1024, 2048, 4096])
+@pytest.mark.parametrize("cells", [
+    lambda e, u: e,              # the smallest line: the tile wraps around it once
+    lambda e, u: e + 1,
+    lambda e, u: 4 * u,          # whole pairs, to the cell (periodic)
+    lambda e, u: 4 * u + 1,      # a tile with one cell, and no partner
+    lambda e, u: 9 * e + 77,
+])
+def test_lines_in_wide_tiles(monkeypatch, cells, edge, boundary):
+    monkeypatch.setenv("FFS_WIDE_TILE", str(edge))
+    plan, err = _line(cells(edge, edge - 2 * 2 * 21), 21, boundary, 2)
+    assert plan.info["tile"] == edge and plan.info["passes"] == 1 and err <= TOL
+
+
+@pytest.mark.parametrize("n,T,radius,in_place,offset", [
+    (30011, 85, 1, False, 1),   # boxes of 255 staged cells, 8-byte-aligned buffers
+    (30011, 100, 1, True, 0),   # 300
+    (30011, 170, 1, False, 0),  # 510
+    (30011, 60, 3, True, 1),    # 540: past a warp's 16 cells a lane
+    (30011, 40, 5, False, 0),   # a radius without a warp's path
+    (7001, 900, 2, True, 0),    # several passes, the last one shorter
+])
+def test_boxes_beside_line_tiles(monkeypatch, n, T, radius, in_place, offset):
+    monkeypatch.setenv("FFS_WIDE_TILE", "2048")
+    plan, err = _line(n, T, "fixed", radius, in_place, offset)
+    assert plan.info["tile"] == 2048 and err <= TOL

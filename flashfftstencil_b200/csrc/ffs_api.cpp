@@ -538,9 +538,9 @@ static ffs_status create_plan(ffs_plan **out, const ffs_problem *problem, Route 
         for (int k = 0; k < sp.npass_kinds; ++k)
             mem.reserve(&p->dev[k].spec, wide_spectrum_count(sp.wtile));
         mem.reserve(&p->d_wide, (size_t)sp.wchunk * wide_tile_bytes(sp.wtile) / sizeof(double2));
-        if (sp.frame)
-            mem.reserve(&p->d_frame, 2 * frame_cells(sp, sp.pass[0].tau));
     }
+    if (sp.frame || sp.strips)
+        mem.reserve(&p->d_frame, 2 * frame_cells(sp, sp.pass[0].tau));
     if ((e = mem.allocate(&p->d_memory)) != cudaSuccess)
         return bail(e, "plan memory");
     if (sp.wide && (e = wide_spectra(p, roots)) != cudaSuccess)
@@ -633,7 +633,7 @@ static BandWork band_work(const ffs_plan *p, int kind, const double *src, double
 static bool band_goes_first(const ffs_plan *p, const PassSpec &ps)
 {
     const PlanSpec &sp = p->spec;
-    if (sp.form != FFS_FORM_FP64_FFT || sp.dim == 1 || sp.wide || (sp.dim == 3 && sp.tile == 32))
+    if (sp.form != FFS_FORM_FP64_FFT || sp.dim == 1 || sp.wide || sp.strips || (sp.dim == 3 && sp.tile == 32))
         return true;
     const int64_t slots = sp.dim == 2 ? std::min<int64_t>(ps.nitems, p->num_sms) : fft3d_grid(ps.nitems, p->num_sms);
     const int64_t tail = ps.nitems % slots;
@@ -845,7 +845,7 @@ static ffs_status run_pass(const ffs_plan *p, int kind, const double *src, doubl
         {
             LaunchMark mark(p, bs, 1);
             cudaError_t e;
-            if (sp.frame) {
+            if (sp.frame || sp.strips) {
                 e = frame_pass(p, kind, src, dst, bs);
             } else {
                 BandWork b = band_work(p, kind, src, dst);
@@ -1368,8 +1368,9 @@ extern "C" ffs_status ffs_plan_get_info(const ffs_plan *plan, ffs_plan_info *inf
     const PlanSpec &sp = plan->spec;
     size_t work = plan->d_work ? sp.cells * sizeof(double) : 0;
     if (sp.wide)
-        work += (size_t)sp.wchunk * wide_tile_bytes(sp.wtile) +
-                (sp.frame ? 2 * frame_cells(sp, sp.pass[0].tau) * sizeof(double) : 0);
+        work += (size_t)sp.wchunk * wide_tile_bytes(sp.wtile);
+    if (sp.frame || sp.strips)
+        work += 2 * frame_cells(sp, sp.pass[0].tau) * sizeof(double);
     info->work_bytes = (int64_t)work;
     return FFS_OK;
 }

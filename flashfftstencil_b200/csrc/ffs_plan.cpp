@@ -611,6 +611,23 @@ double frame_cost(const PlanSpec &sp, int tau, double *busy)
     return n * (launch + kMarchLaunchSeconds);
 }
 
+// Whether the one-SM tiles' band is stepped on the frame too (the same sums in the same order), rather
+// than by a block per box: the boxes' halos are r tau wide on both sides, so past a depth of 16 cells
+// they step little else, and from 8 on a long frame has more of them than SMs (us a solve, boxes / frame:
+// 1536 x 1024, Box2D9P, T = 12 58.8 / 51.5, Box2D25P, T = 4 43.3 / 41.1, T = 12 123.6 / 103.7 in FP64;
+// 4096 x 2048, Box2D25P, T = 12 in 128 x 128 tiles 288 / 197; 200 x 150, Box2D9P, T = 20 37.1 / 24.8).
+// A short or shallow frame costs a second launch or as much as the boxes: 200 x 150, T = 12 16.4 / 18.7;
+// 1536 x 1024, T = 4 27.1 / 29.0.
+bool strips_win(const PlanSpec &sp)
+{
+    if (march_max_tau(sp.radius, sp.star) == 0 || sp.n[0] >= 1 << 30 || sp.n[1] >= 1 << 30)
+        return false;
+    PassSpec ps;
+    geometry(sp, sp.tau, &ps);
+    const int depth = sp.radius * sp.tau;
+    return ps.nitems > 0 && (depth >= 16 || (depth >= 8 && sp.n[0] + sp.n[1] >= 1024));
+}
+
 // ---- wide tiles ----
 
 constexpr int kWideEdges[] = {256, 512, 1024, 2048};
@@ -1464,6 +1481,9 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
         return bad(FFS_ERR_UNSUPPORTED, "stencil radius too large for the tile");
     sp.npass_kinds = (sp.tau_last != sp.tau) ? 2 : 1;
     sp.last_kind = sp.npass_kinds - 1;
+    if (!sp.wide && !sp.direct && sp.dim == 2 && sp.boundary == FFS_BOUNDARY_FIXED &&
+        route != kRouteNoWide)
+        sp.strips = strips_win(sp);
     sp.est_seconds = 0.0;
     for (int k = 0; k < sp.npass_kinds; ++k) {
         const int tau = k == 0 ? sp.tau : sp.tau_last;

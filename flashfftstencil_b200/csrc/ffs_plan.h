@@ -59,6 +59,7 @@ struct PlanSpec {
     bool blocks = false;         // 2-D: by blocks (ffs_step.cu), else by marching warps (ffs_march.cu)
     int line_k = 0;              // 1-D: cells per lane (ffs_line.cu)
     bool frame = false;          // the wide tiles' band is stepped by ffs_step.cu (no band boxes)
+    bool strips = false;         // so is the band of the one-SM tiles (its boxes are for batches)
     bool star = false;           // 2-D: all taps on the axes
     int tau = 0, tau_last = 0, passes = 0;
     int npass_kinds = 0, last_kind = 0;

@@ -140,3 +140,26 @@ def test_boxes_beside_line_tiles(monkeypatch, n, T, radius, in_place, offset):
     monkeypatch.setenv("FFS_WIDE_TILE", "2048")
     plan, err = _line(n, T, "fixed", radius, in_place, offset)
     assert plan.info["tile"] == 2048 and err <= TOL
+
+
+@pytest.mark.parametrize("form,tile", [("fp64", 0), ("fp64_fft", 64), ("fp64_fft", 128), ("ozaki", 0)])
+@pytest.mark.parametrize("ext,T,radius,in_place,offset", [
+    ((200, 150), 16, 1, False, 0),   # the shallowest frame of a short grid, two launches
+    ((201, 149), 20, 1, True, 1),    # odd, in place, 8-byte aligned
+    ((700, 324), 8, 1, False, 0),    # the shallowest of a long one, one launch
+    ((131, 907), 4, 2, False, 1),
+    ((310, 260), 33, 2, True, 0),    # several passes, the last one shorter
+    ((90, 75), 32, 1, False, 0),     # the exact window is small, the strips overlap
+])
+def test_band_of_one_sm_tiles_on_a_frame(ext, T, radius, in_place, offset, form, tile):
+    import torch
+    w = seeded_weights(2, radius, 3)
+    plan = ffs.Plan(2, None, ext, T, weights=w, radius=radius, boundary="fixed", form=form, tile=tile)
+    x = seeded_grid((ext[1], ext[0]), 4)
+    buf = torch.empty(x.size + offset, dtype=torch.float64, device="cuda")
+    d = buf[offset:].view(x.shape)
+    d.copy_(torch.from_numpy(x))
+    out = d if in_place else torch.full_like(d, float("nan"))
+    plan.run(d, out)
+    torch.cuda.synchronize()
+    assert rel_errors(out.cpu().numpy(), oracle.run(x, w, radius, T, oracle.FIXED))[0] <= TOL

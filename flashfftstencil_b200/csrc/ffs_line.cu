@@ -1,9 +1,10 @@
 // Direct FP64 time stepping of 1-D grids: a warp holds a piece of the line in registers and steps it
 // many times.
 //
-// Where: short runs, and lines of up to some 10^5 cells.  The 4096-point tile's launch takes 14 us
-// however few cells there are (copies, three dependent passes of DFT lines, stores); a step here is one
-// exchange between neighbouring lanes and (2r+1) multiply-adds per cell.
+// Where: short runs, and lines of up to some 10^5 cells.  A tile's launch takes 14 us (4096 cells in
+// shared memory) or 10.6 (ffs_wide.cu) however few cells there are; a step here is one exchange between
+// neighbouring lanes and (2r+1) multiply-adds per cell: 10000 cells, radius 2, T = 16 14.4 -> 7.8 us,
+// 2.5 M cells, T = 3 37.3 -> 12.7.
 //
 // A warp owns 32 K consecutive cells, K per lane, of which the outer r steps on either side are margin
 // (none at a fixed face, where the ring holds).  Per step a lane gets the r cells beyond each end of its

@@ -2,7 +2,7 @@
 // down the rows.
 //
 // Where: short runs (few steps between two uses of a grid), where tau (2r+1)^2 multiply-adds
-// per cell cost less than two transforms, and the fixed boundary's band of the wide tiles.
+// per cell cost less than two transforms (Star2D9P 1999 x 2047, T = 4: 64 x 64 tiles 82 us, this 39).
 //
 // A warp owns a strip of 32 K columns, K consecutive ones per lane, and reads the region's rows
 // in order.  Level s (0-based) turns row y of step s into row y - r of step s + 1: row y adds its

@@ -2,7 +2,7 @@
 // z planes.
 //
 // Where: most 3-D runs.  The 16^3 tile's transforms keep (12 / 16)^3 = 0.42 of their points at two
-// fused steps: Box3D27P 512^3 takes 768 us a step that way, Heat-3D 740; one direct step 515 and 396
+// fused steps: Box3D27P 512^3 takes 768 us a step that way, Heat-3D 740; one direct step 450 to 500 and 396
 // (HBM alone: 323).
 //
 // A block of 256 threads owns a 64 x 32 tile of a plane, a thread one column of kRows rows.  Planes (the

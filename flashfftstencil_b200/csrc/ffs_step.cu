@@ -1,11 +1,11 @@
 // Direct FP64 time stepping of 2-D regions by blocks that hold their tile in registers: many
 // steps of a few cells.
 //
-// Where: the fixed boundary's frame of the wide tiles and small grids stepped directly, where a
-// launch is bound by the length of its units.  The marching kernel (ffs_march.cu) has more useful
-// cells per multiply-add on large grids, but its warps walk 2 r tau rows before their first output
-// and leave most of the GPU idle on a strip: 8 launches of 4 steps on the frame of 2048^2 took
-// 170 us.
+// Where: the fixed boundary's frame of the wide tiles, deep bands of the one-SM tiles, and small grids
+// stepped directly (300 x 260, T = 12: 14.4 -> 12.3 us), where a launch is bound by the length of its
+// units.  The marching kernel (ffs_march.cu) has more useful cells per multiply-add on large grids, but
+// its warps walk 2 r tau rows before their first output and leave most of the GPU idle on a strip: 8
+// launches of 4 steps on the frame of 2048^2 took 170 us (a whole solve with this kernel 113).
 //
 // A block of kWarps warps holds a tile of 32 K columns x M kWarps rows: a lane K consecutive columns
 // of the warp's M rows.  Per step a warp leaves its first and last r rows in shared memory (two

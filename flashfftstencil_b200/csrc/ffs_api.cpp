@@ -1531,7 +1531,8 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
             const float mn = time_plan(p);
             if (mn < best) {
                 best = mn;
-                arg = tau;
+                if (!arg) // a plan given the count runs one-SM tiles: theirs is returned
+                    arg = tau;
                 arg_tile = route == kRouteWide ? kWideTuned : kDirectTuned;
             }
         }

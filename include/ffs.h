@@ -64,7 +64,7 @@ typedef enum {
 } ffs_boundary;
 
 typedef enum {
-    FFS_FORM_AUTO = 0,      /* fastest FP64-exact form (FP64_FFT) */
+    FFS_FORM_AUTO = 0,      /* fastest FP64 path: FP64_FFT on one-SM or wide tiles, or direct steps */
     FFS_FORM_FP64_DMMA = 1, /* FP64 mma.sync m8n8k4 DFT GEMMs */
     FFS_FORM_OZAKI_I8 = 2,  /* Ozaki split products on INT8 tcgen05/TMEM */
     FFS_FORM_BF16X3 = 3,    /* 3-way BF16 split, FP32 accumulate (~1e-7 work) */
@@ -104,7 +104,10 @@ typedef struct {
                               its cost model); the FP64 butterfly form takes 64 (a pair of real
                               tiles per CTA) or 128 (one real tile per CTA) in 2D and 16 (one CTA
                               per tile pair) or 32 (a four-CTA cluster per pair) in 3D; every other
-                              form has one edge (1D 4096, 2D 64, 3D 16) and accepts only that */
+                              form has one edge (1D 4096, 2D 64, 3D 16) and accepts only that.
+                              With tile == 0 and tau == 0 the FP64 butterfly form may also take
+                              wide tiles (256 .. 2048 cells an axis through a workspace in 2D,
+                              1024 .. 4096 in 1D), and FFS_FORM_AUTO direct stepping */
     int reserved[6];       /* must be zero */
 } ffs_problem;
 
@@ -112,7 +115,8 @@ typedef struct {
     int dim;
     int radius;
     ffs_form form;       /* resolved form */
-    int tile;            /* DFT tile edge n (per dim) */
+    int tile;            /* DFT tile edge n (per dim; the x edge of a wide tile; direct steps: the
+                            x cells of a warp's or block's piece) */
     int halo;            /* halo per side, >= r * tau, even */
     int useful;          /* cropped output edge u = n - 2 * halo */
     int tau;             /* fused steps per full pass */
@@ -120,7 +124,8 @@ typedef struct {
     int passes;          /* number of passes (ceil(T / tau)) */
     int slices;          /* resolved slice count (Ozaki / BF16 forms) */
     int64_t tiles;       /* tiles per pass */
-    int64_t work_bytes;  /* device workspace owned by the plan */
+    int64_t work_bytes;  /* device workspace owned by the plan (one grid, a wide pass's chunk of
+                            transformed tiles of at most 1 GiB, the fixed band's strips) */
     double flops_per_pass;   /* algorithmic DFT-GEMM flops per pass (dense count) */
     double exec_flops_per_pass; /* flops the chosen factorisation executes per pass */
     double hbm_bytes_per_pass;  /* algorithmic HBM bytes per pass (16 B per cell) */
@@ -183,11 +188,14 @@ ffs_status ffs_plan_destroy(ffs_plan *plan);
  * counts with the plan builder's cost model, times the best `candidates`
  * (0 = 6) on the current device with scratch grids and keeps the fastest; for
  * the FP64 butterfly form in 2D and 3D with problem->tile == 0 it does so for
- * both tile edges (64 and 128, 16 and 32) and keeps the faster edge as well.  For
+ * both tile edges (64 and 128, 16 and 32), for the wide tiles and, for FFS_FORM_AUTO,
+ * for direct stepping, and keeps the fastest of them as well.  For
  * an Ozaki problem with slices == 0 it then calibrates the slice count at that
  * step count: it solves a seeded uniform [0, 1) grid of the problem's geometry
  * with the FP64 butterfly form and with 4 .. 8 slices, and keeps the smallest
  * count whose max relative difference is at most 1e-12 / 1.5 (8 if none is).
+ * best_tau is the fastest count of the form's one-SM tiles, which a plan with that
+ * problem->tau runs; best_ms the time of the fastest choice, which one with tau == 0 takes.
  * The choices go into the process-wide tuning table -- also appended to the
  * file named by FFS_TUNE_CACHE, read back on first use -- keyed by problem class
  * (form, slice count, tile edge, dim, taps, boundary, T, log2 extents);

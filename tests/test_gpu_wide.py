@@ -163,3 +163,10 @@ def test_band_of_one_sm_tiles_on_a_frame(ext, T, radius, in_place, offset, form,
     plan.run(d, out)
     torch.cuda.synchronize()
     assert rel_errors(out.cpu().numpy(), oracle.run(x, w, radius, T, oracle.FIXED))[0] <= TOL
+
+
+def test_autotune_returns_a_count_for_one_sm_tiles():
+    """A plan given the returned count runs that many steps a pass, whichever route was the fastest."""
+    tau, ms = ffs.autotune(2, "Box2D25P", (1100, 1000), 120, boundary="periodic", form="auto", candidates=2)
+    info = ffs.Plan(2, "Box2D25P", (1100, 1000), 120, boundary="periodic", form="auto", tau=tau).info
+    assert info["tau"] == tau and info["tile"] in (64, 128) and ms > 0

@@ -666,7 +666,7 @@ def run_batch_workload(args):
                                    "32-256), T uniform 1..64, boundary fixed/periodic at random",
                        "form": form,
                        "execution": "one CUDA graph per replay: FP64-DMMA plans in one persistent kernel, plans "
-                                    "of the other forms as their own launches on 8 parallel graph branches",
+                                    "of the other forms as their own launches on 16 parallel graph branches",
                        "cell_steps": cells, "problems": len(specs)},
             "per_problem_launches": {"value": cells / (ms_plain * 1e-3) / 1e9, "ms_per_step": ms_plain},
             "speedup_vs_per_problem": ms_plain / ms_batch,
@@ -756,10 +756,11 @@ def measure_targets(ffs, torch, steps, warmup, with_oracle):
         for form, sl in TARGET_FORMS:
             # Ozaki with slices 0: the autotuner calibrates the slice count against the FP64 form
             key = FORMS[form][0] + ((f"_s{sl}" if sl else "_auto") if form == "ozaki" else "")
-            tau = ffs.autotune(si.dim, None, ext, T, candidates=4, weights=w, radius=si.radius, boundary=bnd,
-                               form=form, slices=sl)[0]
+            # (the plan takes its choice from the tuning table: tau = 0)
+            ffs.autotune(si.dim, None, ext, T, candidates=4, weights=w, radius=si.radius, boundary=bnd,
+                         form=form, slices=sl)
             plan = ffs.Plan(si.dim, None, ext, T, weights=w, radius=si.radius, boundary=bnd, form=form,
-                            slices=sl, tau=tau)
+                            slices=sl)
             d_out = plan.run(d_in)
             torch.cuda.synchronize()
             acc = rel_errors(d_out.cpu().numpy(), ref) if ref is not None else (None, None)
@@ -965,8 +966,8 @@ def main():
             head_plan = plan
         else:
             plan.close()
-    # the butterfly form's other 2D tile edge (64 x 64 pairs or one real 128 x 128 tile per CTA),
-    # beside the plan builder's choice for this grid
+    # the butterfly form's largest one-SM tile edge (64 x 64 pairs or one real 128 x 128 tile per CTA)
+    # that the plan builder did not choose for this grid, beside its choice
     other_edge = None
     if "fp64_fft" in results and not pg:
         edge = 64 if results["fp64_fft"]["info"]["tile"] == 128 else 128
@@ -1097,7 +1098,14 @@ def main():
     peak = pipe_peak[args.form]
     pipe = {"achieved": achieved, "peak": peak, "unit": "TOPS" if args.form == "ozaki" else "TFLOP/s",
             "frac": achieved / peak if peak else None}
-    if args.form == "fp64_fft":
+    wide = args.form == "fp64_fft" and info["tile"] >= 256
+    if wide:
+        # wide tiles: three kernels per pass over a workspace in HBM.  Reported against the pass's own
+        # 16 bytes per cell; each tile point also crosses HBM twice more between the kernels
+        roofline = {"bound": "hbm", "achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
+                    "frac": hbm_achieved / hbm_peak if hbm_peak else None,
+                    "fp64_pipe": dict(pipe, peak_source="fma.rn.f64 loop")}
+    elif args.form == "fp64_fft":
         # no tensor pipe: the binding roof is shared-memory bandwidth, the FP64 pipe is reported beside it
         if info["tile"] == 128:
             smem_bytes = fft2d128_smem_bytes_per_tile(info["useful"]) * info["tiles"]
@@ -1119,7 +1127,8 @@ def main():
                 "traffic_source": (f"{tr.get('source')} (profiles/{TRAFFIC_FILES[(args.form, info['tile'])]}, captured on "
                                    f"commit {tr.get('captured_on', 'unrecorded')}, not measured in this run)")
                                   if tr else None,
-                "kernel": ("ffst::fft2d128::fft2d128_kernel" if args.form == "fp64_fft" and info["tile"] == 128
+                "kernel": ("ffst::wide::rows_fwd_kernel, cols_kernel, rows_inv_kernel (one pass)" if wide
+                           else "ffst::fft2d128::fft2d128_kernel" if args.form == "fp64_fft" and info["tile"] == 128
                            else kern_name[args.form]),
                 "peak_source": "measured in this run: " + peaks["how"],
                 "flops_per_launch": info["exec_flops_per_pass"],
@@ -1135,6 +1144,8 @@ def main():
                 "hbm": {"achieved_gbs": hbm_achieved, "peak_gbs": hbm_peak, "frac": hbm_achieved / hbm_peak,
                         "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks_file else "fallback"}})
     launches = prof["tile_launches"] + prof["band_launches"]
+    if wide:  # a traced pass is three kernels and the band's strips, stepped at most 11 steps per launch
+        launches = 3 * prof["tile_launches"] + -(-info["tau"] // 11) * prof["band_launches"]
     # on several GPUs the same headline grid is also solved split into slabs over the ranks
     # (strong scaling, NCCL ghost exchange per pass), reported beside the replicas value
     decomposed = None

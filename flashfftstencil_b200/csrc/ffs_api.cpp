@@ -409,6 +409,15 @@ static void release(ffs_plan *p)
     delete p;
 }
 
+// A copy from pageable memory may return while its last part is still on the way from the driver's
+// staging buffer, and only work on the legacy stream is ordered behind it; plans and batches run on
+// any stream, so the copy is waited for.
+static cudaError_t upload(void *dst, const void *src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(nullptr);
+}
+
 // A plan's device memory is one allocation, filled by one copy: each cudaMalloc of 1 MB to 180 MB
 // takes 0.4 ms, and a plan has up to a dozen arrays.  Collects the arrays with their contents
 // first (each starts on a 256-byte boundary), then the buffers without.
@@ -444,7 +453,7 @@ struct PlanMemory {
     {
         cudaError_t e = cudaMalloc(base, size);
         if (e == cudaSuccess)
-            e = cudaMemcpy(*base, image.data(), image.size(), cudaMemcpyHostToDevice);
+            e = upload(*base, image.data(), image.size());
         if (e != cudaSuccess)
             return e;
         for (const Piece &q : pieces)
@@ -1741,8 +1750,8 @@ static ffs_status build_queue(ffs_batch *b, const double *const *ins, double *co
     CUDA_TRY(cudaMalloc(&b->d_stages, stages.size() * sizeof(BatchStage)));
     CUDA_TRY(cudaMalloc(&b->d_start, start.size() * sizeof(int64_t)));
     CUDA_TRY(cudaMalloc(&b->d_done, stages.size() * sizeof(int)));
-    CUDA_TRY(cudaMemcpy(b->d_stages, stages.data(), stages.size() * sizeof(BatchStage), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(b->d_start, start.data(), start.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
+    CUDA_TRY(upload(b->d_stages, stages.data(), stages.size() * sizeof(BatchStage)));
+    CUDA_TRY(upload(b->d_start, start.data(), start.size() * sizeof(int64_t)));
     return FFS_OK;
 }
 

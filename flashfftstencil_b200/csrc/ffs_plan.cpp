@@ -509,7 +509,9 @@ double tile_route_cost(const PlanSpec &sp)
 
 double pick_direct3(PlanSpec *sp, bool forced)
 {
-    if (sp->radius != 1 || sp->n[0] >= 1 << 30 || sp->n[2] >= 1 << 30 || sp->n[0] * sp->n[1] >= 1ll << 31)
+    // (an open face's stepped cells end at +-2^30; offsets in a plane are 32-bit)
+    if (sp->radius != 1 || sp->n[0] >= 1 << 30 || sp->n[1] >= 1 << 30 || sp->n[2] >= 1 << 30 ||
+        sp->n[0] * sp->n[1] >= 1ll << 31)
         return INFINITY;
     sp->tau = sp->tau_last = 1;
     sp->passes = sp->T;

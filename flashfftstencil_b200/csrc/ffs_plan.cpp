@@ -357,8 +357,14 @@ int max_tau(const PlanSpec &sp)
     return tau_max;
 }
 
+// Whether the tile has cells left between the halos of tau steps (a 16^3 tile has none at radius 7
+// and 8; the geometry divides by their number).
+bool tile_holds(const PlanSpec &sp, int tau) { return sp.tile > 2 * round_even(sp.radius * tau); }
+
 double model_cost(const PlanSpec &sp, int tau)
 {
+    if (!tile_holds(sp, tau))
+        return INFINITY;
     PassSpec ps;
     geometry(sp, tau, &ps);
     const int passes = (sp.T + tau - 1) / tau;
@@ -384,11 +390,9 @@ void pick_tau(PlanSpec *sp, int tau_override)
     }
     if (!best) {
         double best_cost = 1e300;
+        best = 1; // (of an edge too small for the radius, which the caller refuses)
         for (int tau = 1; tau <= tau_max; ++tau) {
-            PassSpec ps;
-            geometry(*sp, tau, &ps);
-            const int passes = (sp->T + tau - 1) / tau;
-            const double c = passes * pass_cost(*sp, ps, 148);
+            const double c = model_cost(*sp, tau);
             if (c < best_cost * (1 - 1e-9)) {
                 best_cost = c;
                 best = tau;
@@ -491,7 +495,7 @@ double march3_cost(const PlanSpec &sp)
 double tile_route_cost(const PlanSpec &sp)
 {
     double c = model_cost(sp, sp.tau), more = 0.0;
-    if (sp.form != FFS_FORM_FP64_FFT)
+    if (sp.form != FFS_FORM_FP64_FFT || !tile_holds(sp, sp.tau))
         return c;
     if (sp.dim == 3 && sp.tile == 16)
         more = 3e-6;

@@ -1,0 +1,25 @@
+"""Calls whose route the plan builder decides at the edge of a kernel's range, against the oracle."""
+import pytest
+
+import flashfftstencil_b200 as ffs
+import oracle
+from tests.helpers import rel_errors, seeded_grid, seeded_weights
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # the FP64 forms' tolerance
+
+
+@pytest.mark.parametrize("boundary", ["fixed", "periodic"])
+@pytest.mark.parametrize("radius", [7, 8])
+def test_largest_radii_in_3d(radius, boundary):
+    """Halos of 8 cells a side leave a 16^3 tile nothing and a 32^3 tile half its edge."""
+    import torch
+    ext = (40, 36, 33)
+    w = seeded_weights(3, radius, 2)
+    plan = ffs.Plan(3, None, ext, 2, weights=w, radius=radius, boundary=boundary, form="auto")
+    assert plan.info["tile"] == 32
+    x = seeded_grid(tuple(reversed(ext)), 3)
+    y = plan.run(torch.from_numpy(x).cuda())
+    torch.cuda.synchronize()
+    ref = oracle.run(x, w, radius, 2, oracle.FIXED if boundary == "fixed" else oracle.PERIODIC)
+    assert rel_errors(y.cpu().numpy(), ref)[0] <= TOL

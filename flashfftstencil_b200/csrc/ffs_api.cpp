@@ -1529,8 +1529,11 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
             arg_tile = at.tile;
         }
     }
+    if (tiles.size() > 1 && arg)
+        tune_record(tile_key(spec), arg_tile);
     // the model's choice of wide tile, and of direct stepping, against the best edge
     const bool routes = problem->tile == 0 && problem->tau == 0 && spec.form == FFS_FORM_FP64_FFT;
+    int arg_route = kTilesTuned;
     if (routes)
         for (Route route : {kRouteWide, kRouteDirect}) {
             ffs_plan *p = nullptr;
@@ -1542,7 +1545,7 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
                 best = mn;
                 if (!arg) // a plan given the count runs one-SM tiles: theirs is returned
                     arg = tau;
-                arg_tile = route == kRouteWide ? kWideTuned : kDirectTuned;
+                arg_route = route == kRouteWide ? kWideTuned : kDirectTuned;
             }
         }
     cudaEventDestroy(e0);
@@ -1552,8 +1555,8 @@ extern "C" ffs_status ffs_autotune(const ffs_problem *problem, int candidates, i
         cudaFree(dout);
         return fail(FFS_ERR_INTERNAL, "ffs_autotune: no candidate could run");
     }
-    if (tiles.size() > 1 || routes)
-        tune_record(tile_key(spec), arg_tile);
+    if (routes)
+        tune_record(route_key(spec, problem->form == FFS_FORM_AUTO), arg_route);
     if (spec.form == FFS_FORM_OZAKI_I8 && problem->slices == 0) {
         // the slice count at the chosen fused step count, recorded with that count
         ffs_problem q = *problem;

@@ -1183,8 +1183,7 @@ std::string tune_key(const PlanSpec &sp)
     return buf;
 }
 
-// The same class without the tile edge: key of the measured tile choice of the 3D
-// butterfly form.
+// The same class without the tile edge: key of the measured edge of the butterfly form's one-SM tiles.
 std::string tile_key(const PlanSpec &sp)
 {
     char buf[256];
@@ -1194,6 +1193,14 @@ std::string tile_key(const PlanSpec &sp)
     snprintf(buf, sizeof(buf), "E.f%d.d%d.r%d.k%zu.b%d.o%d.T%d.n%d_%d_%d", (int)sp.form, sp.dim, sp.radius,
              sp.taps.size(), (int)sp.boundary, sp.open_faces, sp.T, lg[0], lg[1], lg[2]);
     return buf;
+}
+
+// The same class for the route (one-SM tiles, wide tiles or direct steps).  The automatic form and the
+// butterfly form by name have an entry each: only the first may step directly, so a route measured for
+// one was not chosen among the other's.
+std::string route_key(const PlanSpec &sp, bool automatic)
+{
+    return (automatic ? "RA." : "R.") + tile_key(sp).substr(2);
 }
 
 // The same class without the slice count: key of the calibrated Ozaki slice count.
@@ -1449,36 +1456,39 @@ ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why
     }
     pick_tau(&sp, p.tau);
     // wide tiles and direct stepping: only where the caller left both the edge and the step count
-    // open; a measured choice for the class wins over the model, as for the edges
+    // open.  Direct stepping is the automatic form's; the butterfly form asked for by name stays that.
     if (p.tile == 0 && p.tau == 0 && sp.T > 0 && sp.form == FFS_FORM_FP64_FFT) {
-        int measured = route == kRouteAuto ? tune_lookup(tile_key(sp)) : 0;
-        if (sp.dim == 1 && measured == 0 && route == kRouteAuto && tune_lookup(tune_key(sp)) > 0)
-            measured = sp.tile; // a table written before 1-D had two routes
-        const bool edge_measured = measured > kDirectTuned; // 4096 (1D), 64, 128 (2D), 16, 32 (3D)
-        double best = route >= kRouteWide || measured == kWideTuned || measured == kDirectTuned ? INFINITY
-                                                                                              : tile_route_cost(sp);
-        if (edge_measured)
-            best = 0.0;
-        PlanSpec w = sp, d = sp;
-        if (route != kRouteNoWide && route != kRouteDirect && !edge_measured && measured != kDirectTuned) {
-            const double c = pick_wide(&w);
-            if (c < best) {
-                best = c;
-                sp = std::move(w);
-                sp.wide = true;
-                sp.tile = sp.wtile[0];
+        const bool may_step = p.form == FFS_FORM_AUTO && direct_override() != "0";
+        auto choose = [&](bool tiles, bool wide, bool direct) { // the cheapest modelled of these that fits
+            double best = tiles ? tile_route_cost(sp) : INFINITY;
+            PlanSpec w = sp, d = sp;
+            if (wide) {
+                const double c = pick_wide(&w);
+                if (c < best) {
+                    best = c;
+                    sp = std::move(w);
+                    sp.wide = true;
+                    sp.tile = sp.wtile[0];
+                }
             }
-        }
-        // direct stepping is the automatic form's; the butterfly form asked for by name stays that
-        if (p.form == FFS_FORM_AUTO && route != kRouteWide && !edge_measured && measured != kWideTuned &&
-            direct_override() != "0") {
-            const double c = pick_direct(&d);
-            if (c < best) {
-                best = c;
-                sp = std::move(d);
-                sp.direct = true;
-                sp.tile = sp.dim == 1 ? 32 * sp.line_k : sp.dim == 2 ? 128 : 64;
+            if (direct) {
+                const double c = pick_direct(&d);
+                if (c < best) {
+                    best = c;
+                    sp = std::move(d);
+                    sp.direct = true;
+                    sp.tile = sp.dim == 1 ? 32 * sp.line_k : sp.dim == 2 ? 128 : 64;
+                }
             }
+        };
+        // a measured choice for the class wins over the model, where it fits this problem
+        const int measured = route == kRouteAuto ? tune_lookup(route_key(sp, p.form == FFS_FORM_AUTO)) : 0;
+        if (measured != kTilesTuned) {
+            if (route == kRouteWide || route == kRouteDirect || measured == kWideTuned || measured == kDirectTuned)
+                choose(false, route == kRouteWide || measured == kWideTuned,
+                       may_step && (route == kRouteDirect || measured == kDirectTuned));
+            if (!sp.wide && !sp.direct && route < kRouteWide)
+                choose(true, route != kRouteNoWide, may_step);
         }
     }
     if ((route == kRouteWide && !sp.wide) || (route == kRouteDirect && !sp.direct))

@@ -80,8 +80,8 @@ enum Route {
 // spectra and tables are not computed (fast describe path).
 ffs_status build_plan_spec(const ffs_problem &p, PlanSpec *out, std::string *why, bool with_data = true,
                            Route route = kRouteAuto);
-// Values of tile_key's entry for a class whose measured best is not a one-SM tile edge.
-constexpr int kWideTuned = 1, kDirectTuned = 2;
+// Values of route_key's entry.
+constexpr int kWideTuned = 1, kDirectTuned = 2, kTilesTuned = 3;
 // Wide tiles: the line transform's twiddles of an axis of n points, and its roots
 // exp(+2 pi i m / n) as pairs of doubles for the spectrum kernel.
 std::vector<double2> wide_twiddles(int n, int axis);
@@ -106,11 +106,13 @@ std::vector<int> tau_candidates(const ffs_problem &p, int count);
 
 // Measured-tuning table: key of a problem class, and lookup/record of its best tau;
 // slice_key names the class without its slice count, whose entry is the calibrated
-// Ozaki slice count, and tile_key the class without its tile edge, whose entry is the
-// measured tile edge of the 3D butterfly form (ffs_autotune).
+// Ozaki slice count, tile_key the class without its tile edge, whose entry is the
+// measured edge of the butterfly form's one-SM tiles, and route_key the class whose entry
+// is the measured route, for plans of the automatic form or of the butterfly form by name.
 std::string tune_key(const PlanSpec &sp);
 std::string slice_key(const PlanSpec &sp);
 std::string tile_key(const PlanSpec &sp);
+std::string route_key(const PlanSpec &sp, bool automatic);
 int tune_lookup(const std::string &key);
 void tune_record(const std::string &key, int value);
 

@@ -198,7 +198,9 @@ ffs_status ffs_plan_destroy(ffs_plan *plan);
  * problem->tau runs; best_ms the time of the fastest choice, which one with tau == 0 takes.
  * The choices go into the process-wide tuning table -- also appended to the
  * file named by FFS_TUNE_CACHE, read back on first use -- keyed by problem class
- * (form, slice count, tile edge, dim, taps, boundary, T, log2 extents);
+ * (form, slice count, tile edge, dim, taps, boundary, T, log2 extents; the choice
+ * between one-SM tiles, wide tiles and direct steps separately for FFS_FORM_AUTO and
+ * for FFS_FORM_FP64_FFT, since only the first may step directly);
  * ffs_plan_create consults it when problem->tau == 0 (fused steps), when
  * problem->tile == 0 (tile edge) and, for the Ozaki form, when
  * problem->slices == 0 (slice count; 7 when the class was never calibrated). */

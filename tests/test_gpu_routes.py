@@ -23,3 +23,19 @@ def test_largest_radii_in_3d(radius, boundary):
     torch.cuda.synchronize()
     ref = oracle.run(x, w, radius, 2, oracle.FIXED if boundary == "fixed" else oracle.PERIODIC)
     assert rel_errors(y.cpu().numpy(), ref)[0] <= TOL
+
+
+def test_tuning_one_form_leaves_the_other_its_route():
+    """auto may step directly, the butterfly form by name may not: what was measured for one does not bind the other."""
+    for dim, shape, ext, T, boundary in ((3, "Box3D27P", (150, 140, 130), 6, "periodic"), (2, "Box2D9P", (700, 600), 40, "periodic"),
+                                         (1, "Heat-1D", (40_000,), 21, "periodic")):
+        def route(form):  # (the one-SM tiles' step count is the two forms' together)
+            i = ffs.describe(dim, shape, ext, T, boundary=boundary, form=form)
+            wide = i["tile"] in ((1024, 2048) if dim == 1 else (256, 512, 1024, 2048))
+            return "direct" if i["tiles"] == 1 else "wide" if wide else "tiles"
+        model = route("auto")
+        ffs.autotune(dim, shape, ext, T, boundary=boundary, form="fp64_fft", candidates=2)
+        named = route("fp64_fft")
+        assert route("auto") == model and named != "direct", (dim, model, named)
+        ffs.autotune(dim, shape, ext, T, boundary=boundary, form="auto", candidates=2)
+        assert route("fp64_fft") == named, (dim, model, named)

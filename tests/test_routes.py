@@ -1,8 +1,14 @@
 """The plan builder's choice between the one-SM tiles, wide tiles and direct steps (describe(), no GPU)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import flashfftstencil_b200 as ffs
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _direct(info):
@@ -34,3 +40,53 @@ def test_radius_without_room_in_a_16_tile(radius, boundary):
             with pytest.raises(ffs.FFSError) as e:
                 ffs.describe(3, None, (60, 50, 40), 2, tau=tau, **refused, **kw)
             assert e.value.status == ffs.ERR_UNSUPPORTED
+
+
+# (dim, shape, extents, T, boundary), and the class as the table names it
+VOLUME = (3, "Box3D27P", (512, 512, 512), 16, "fixed")
+PLATE = (2, "Box2D9P", (4096, 4096), 32, "periodic")
+SMALL = (2, "Box2D9P", (100, 100), 40, "periodic")  # below the wide tiles' least side
+VOLUME_CLASS = "f4.d3.r1.k27.b1.o0.T16.n9_9_9"
+PLATE_CLASS = "f4.d2.r1.k9.b0.o0.T32.n12_12_0"
+SMALL_CLASS = "f4.d2.r1.k9.b0.o0.T40.n7_7_0"
+
+
+def _routes(table, tmp_path):
+    """Route ("tiles", "wide", "direct") of each grid for both forms, by a process with this table."""
+    cache = tmp_path / "table"
+    cache.write_text("".join(line + "\n" for line in table))
+    code = ("import sys; sys.path.insert(0, %r); import flashfftstencil_b200 as f\n"
+            "for g in %r:\n"
+            "    for form in ('auto', 'fp64_fft'):\n"
+            "        i = f.describe(*g[:4], boundary=g[4], form=form)\n"
+            "        wide = i['tile'] >= 256\n"
+            "        print('wide' if wide else 'direct' if i['tiles'] == 1 else 'tiles')" %
+            (ROOT, [VOLUME, PLATE, SMALL]))
+    env = {k: v for k, v in os.environ.items() if not k.startswith("FFS_")}
+    r = subprocess.run([sys.executable, "-c", code], env=dict(env, FFS_TUNE_CACHE=str(cache)), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr
+    got = r.stdout.split()
+    return {name: tuple(got[2 * k:2 * k + 2]) for k, name in enumerate(("volume", "plate", "small"))}
+
+
+MODEL = {"volume": ("direct", "tiles"), "plate": ("wide", "wide"), "small": ("tiles", "tiles")}
+
+
+@pytest.mark.parametrize("table,changed", [
+    ([], {}),
+    # a measured one-SM edge ranks the edges only: it was not timed against the other routes
+    (["E." + VOLUME_CLASS + " 16", "E." + PLATE_CLASS + " 128"], {}),
+    # entries of either form's tuning by an earlier version, whose key did not tell them apart
+    (["E." + VOLUME_CLASS + " 2", "E." + PLATE_CLASS + " 2"], {}),
+    # each form's measured route is its own
+    (["RA." + VOLUME_CLASS + " 3"], {"volume": ("tiles", "tiles")}),
+    (["R." + VOLUME_CLASS + " 3", "R." + PLATE_CLASS + " 3"], {"plate": ("wide", "tiles")}),
+    (["RA." + PLATE_CLASS + " 2"], {"plate": ("direct", "wide")}),
+    (["RA." + PLATE_CLASS + " 3", "R." + PLATE_CLASS + " 1"], {"plate": ("tiles", "wide")}),
+    # a route that the form may not take, or that does not fit this grid of the class: the model's
+    (["R." + PLATE_CLASS + " 2", "RA." + SMALL_CLASS + " 1", "R." + SMALL_CLASS + " 1"], {}),
+])
+def test_tuned_routes_of_the_two_forms(table, changed, tmp_path):
+    """(auto, fp64_fft by name): tuning one form leaves the other's choice alone."""
+    assert _routes(table, tmp_path) == dict(MODEL, **changed)

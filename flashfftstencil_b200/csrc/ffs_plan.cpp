@@ -533,6 +533,18 @@ double line_cost(const PlanSpec &sp, int k, int steps)
     return std::max(busy, steps * (kLineStepSeconds + kLineCellSeconds * taps * k) + kLineLaunchSeconds);
 }
 
+// Calls use(tau, passes) for the step counts, most at a time, that split T evenly into up to `times` the
+// fewest passes: each count once with its fewest passes, so a plan for 10^9 steps looks at no more of them
+// than one for 1000.
+template <class Use>
+void even_steps(int T, int most, int times, Use use)
+{
+    const int64_t limit = times * ceil_div(T, most);
+    for (int tau = std::min(most, T); tau >= 1 && ceil_div(T, tau) <= limit; --tau)
+        if (ceil_div(T, ceil_div(T, tau)) == tau)
+            use(tau, (int)ceil_div(T, tau));
+}
+
 double pick_direct1(PlanSpec *sp, bool forced)
 {
     double best = INFINITY;
@@ -540,18 +552,16 @@ double pick_direct1(PlanSpec *sp, bool forced)
         const int most = line_max_steps(sp->radius, k);
         if (most == 0)
             continue;
-        const int least = (sp->T + most - 1) / most;
-        for (int passes = least; passes <= std::min(sp->T, 3 * least); ++passes) {
-            const int tau = (sp->T + passes - 1) / passes;
+        even_steps(sp->T, most, 3, [&](int tau, int passes) {
             const double c = passes * line_cost(*sp, k, tau);
             if (c < best) {
                 best = c;
                 sp->line_k = k;
                 sp->tau = tau;
-                sp->passes = (sp->T + tau - 1) / tau;
-                sp->tau_last = sp->T - (sp->passes - 1) * tau;
+                sp->passes = passes;
+                sp->tau_last = sp->T - (passes - 1) * tau;
             }
-        }
+        });
     }
     return forced && best < INFINITY ? 0.0 : best;
 }
@@ -572,9 +582,7 @@ double pick_direct(PlanSpec *sp)
         if (only == (blocks ? "march" : "blocks"))
             continue;
         const int most = blocks ? step_max_steps(r) : march_max_tau(r, sp->star);
-        const int least = (sp->T + most - 1) / most;
-        for (int passes = least; passes <= std::min(sp->T, 2 * least); ++passes) {
-            const int tau = (sp->T + passes - 1) / passes;
+        even_steps(sp->T, most, 2, [&](int tau, int passes) {
             const double U = blocks ? step_width(r, tau) : 1;
             const double c = passes * (blocks ? step_cost(*sp, std::ceil(sp->n[0] / U) * std::ceil(sp->n[1] / U), tau)
                                               : march_cost(*sp, (double)sp->n[0], (double)sp->n[1], tau));
@@ -582,10 +590,10 @@ double pick_direct(PlanSpec *sp)
                 best = c;
                 sp->blocks = blocks;
                 sp->tau = tau;
-                sp->passes = (sp->T + tau - 1) / tau;
-                sp->tau_last = sp->T - (sp->passes - 1) * tau;
+                sp->passes = passes;
+                sp->tau_last = sp->T - (passes - 1) * tau;
             }
-        }
+        });
     }
     return only == "march" || only == "blocks" ? 0.0 : best;
 }

@@ -2,6 +2,7 @@
 import os
 import subprocess
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -90,3 +91,14 @@ MODEL = {"volume": ("direct", "tiles"), "plate": ("wide", "wide"), "small": ("ti
 def test_tuned_routes_of_the_two_forms(table, changed, tmp_path):
     """(auto, fp64_fft by name): tuning one form leaves the other's choice alone."""
     assert _routes(table, tmp_path) == dict(MODEL, **changed)
+
+
+@pytest.mark.parametrize("dim,shape,ext", [(1, "Heat-1D", (10_000,)), (2, "Heat-2D", (300, 260)), (2, "Box2D25P", (300, 260))])
+def test_plans_for_very_many_steps_are_made_at_once(dim, shape, ext):
+    """The step counts looked at are bounded by the kernels' most steps a launch, not by T (9 s for 10^9 steps
+    when every pass count was)."""
+    start = time.perf_counter()
+    for boundary in ("fixed", "periodic"):
+        info = ffs.describe(dim, shape, ext, 10 ** 9, boundary=boundary, form="auto")
+        assert (info["passes"] - 1) * info["tau"] + info["tau_last"] == 10 ** 9
+    assert time.perf_counter() - start < 0.2  # 1 to 10 ms

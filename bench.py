@@ -666,7 +666,7 @@ def run_batch_workload(args):
                                    "32-256), T uniform 1..64, boundary fixed/periodic at random",
                        "form": form,
                        "execution": "one CUDA graph per replay: FP64-DMMA plans in one persistent kernel, plans "
-                                    "of the other forms as their own launches on 16 parallel graph branches",
+                                    "of the other forms as their own launches on 8 parallel graph branches",
                        "cell_steps": cells, "problems": len(specs)},
             "per_problem_launches": {"value": cells / (ms_plain * 1e-3) / 1e9, "ms_per_step": ms_plain},
             "speedup_vs_per_problem": ms_plain / ms_batch,

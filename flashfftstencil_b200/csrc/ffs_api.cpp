@@ -303,7 +303,7 @@ struct ffs_batch {
     uint32_t dep_limit = kDepSpinLimit; // FFS_BATCH_WAIT_POLLS overrides it at creation
     // plans outside the persistent kernel (the butterfly and tensor-core forms) run as
     // their own launches on parallel branches of the graph (created on first capture)
-    static constexpr int kBranches = 16; // a mixed batch of 96: 3.84 ms with 3 or 8, 3.59 with 16, 3.71 with 32
+    static constexpr int kBranches = 8;
     cudaStream_t branch[kBranches] = {};
     cudaEvent_t bfork = nullptr, bjoin[kBranches] = {};
 };
@@ -312,13 +312,12 @@ static cudaError_t ensure_branches(ffs_batch *b)
 {
     if (b->bfork)
         return cudaSuccess;
-    int least = 0, greatest = 0;
-    cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    cudaError_t e = cudaSuccess;
     for (int k = 0; k < ffs_batch::kBranches && e == cudaSuccess; ++k) {
-        // The longest solves come first and so lie on the first branches: their blocks go first.  A solve of
-        // 60 dependent launches otherwise waits at each for the other branches' blocks to drain (4.17 -> 3.86 ms
-        // for that batch).
-        e = cudaStreamCreateWithPriority(&b->branch[k], cudaStreamNonBlocking, std::min(least, greatest + k));
+        // No priorities, here or in the graph: a batch runs at that of the stream it is launched into.  With the
+        // longest solves' branches at the device's greatest, a mixed batch of 96 took 3.7 instead of 4.2 ms, but
+        // ten short kernels on a caller's stream of higher priority waited 8 ms for another batch instead of 0.6.
+        e = cudaStreamCreateWithFlags(&b->branch[k], cudaStreamNonBlocking);
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(&b->bjoin[k], cudaEventDisableTiming);
     }
@@ -1851,7 +1850,7 @@ extern "C" ffs_status ffs_batch_execute(ffs_batch *b, const double *const *ins, 
             return fail(FFS_ERR_CUDA, "batch capture: %s", cudaGetErrorString(e != cudaSuccess ? e : ee));
         }
         b->graph = g;
-        CUDA_TRY(cudaGraphInstantiate(&b->exec, g, cudaGraphInstantiateFlagUseNodePriority));
+        CUDA_TRY(cudaGraphInstantiate(&b->exec, g, 0));
         b->ins.assign(ins, ins + n);
         b->outs.assign(outs, outs + n);
         b->stream = s;

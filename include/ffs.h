@@ -226,7 +226,7 @@ ffs_status ffs_shape_lookup(const char *name, ffs_shape *shape, int *dim, int *r
  * with their own kernels.  The launch sequence is captured in a CUDA graph on
  * the first execute and replayed while the buffer pointers match.  A batch uses
  * its plans' workspaces: do not run one of its plans on its own while the batch
- * may still be running. */
+ * may still be running.  Its kernels run at the priority of `stream`. */
 ffs_status ffs_batch_create(ffs_batch **out, ffs_plan *const *plans, int count);
 ffs_status ffs_batch_execute(ffs_batch *batch, const double *const *d_ins, double *const *d_outs,
                              void *stream);

@@ -144,6 +144,7 @@ ffs_status prepare_device(int dev)
     CUDA_TRY(prepare_march());
     CUDA_TRY(prepare_step());
     CUDA_TRY(prepare_march3());
+    CUDA_TRY(prepare_line());
     CUDA_TRY(prepare_dmma1d());
     CUDA_TRY(prepare_dmma3d());
     CUDA_TRY(prepare_tc2d());

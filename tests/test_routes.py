@@ -102,3 +102,25 @@ def test_plans_for_very_many_steps_are_made_at_once(dim, shape, ext):
         info = ffs.describe(dim, shape, ext, 10 ** 9, boundary=boundary, form="auto")
         assert (info["passes"] - 1) * info["tau"] + info["tau_last"] == 10 ** 9
     assert time.perf_counter() - start < 0.2  # 1 to 10 ms
+
+
+@pytest.mark.parametrize("form", ["auto", "fp64_fft"])
+@pytest.mark.parametrize("edge", [0, 64, 128])
+def test_slab_passes_are_those_of_the_one_sm_tiles(edge, form, tmp_path):
+    """A decomposed solve takes the tuned edge's step counts, or the modelled edge's, whatever the route of one
+    grid; in 1-D those of the 4096-cell tile."""
+    cache = tmp_path / "table"
+    cache.write_text("E.%s %d\n" % (PLATE_CLASS, edge) if edge else "")
+    code = ("import sys; sys.path.insert(0, %r)\n"
+            "import flashfftstencil_b200 as f\n"
+            "from flashfftstencil_b200.slab import SlabPlan\n"
+            "for g, tile in ((%r, %r), ((1, 'Heat-1D', (1 << 20,), 500, 'fixed'), 4096)):\n"
+            "    p = SlabPlan(*g[:4], boundary=g[4], rank=1, world=4, form=%r)\n"
+            "    i = f.describe(*g[:4], boundary=g[4], form=%r, tile=tile)\n"
+            "    print([q.tau for q in p.passes] == [i['tau']] * (i['passes'] - 1) + [i['tau_last']])" %
+            (ROOT, PLATE, edge or 128, form, form))
+    env = {k: v for k, v in os.environ.items() if not k.startswith("FFS_")}
+    r = subprocess.run([sys.executable, "-c", code], env=dict(env, FFS_TUNE_CACHE=str(cache)), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == ["True", "True"]

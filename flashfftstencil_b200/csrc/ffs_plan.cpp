@@ -491,7 +491,8 @@ double march3_cost(const PlanSpec &sp)
 // - 2-D: an odd row length rules TMA out, and the 64 x 64 tiles of a 1999 x 2047 grid took 1.9 times as
 //   long with wrapped plain loads, 1.3 times with clipped ones;
 // - 1-D: a wave takes 10.5 us, not 6 (16.7 M cells 150 us, 44.3 M 404 us, a few thousand 14.8), and a band
-//   whose boxes fit a warp (256 staged cells) hides beside it (2^20, fixed, T = 64: 14.9 us).
+//   of short boxes hides beside it (2^20, fixed, T = 64: 14.9 us).  Boxes of 2 r tau staged cells are one warp's
+//   up to 512, but deeper ones than r tau = 85 were not timed beside these tiles: their band counts in full.
 double tile_route_cost(const PlanSpec &sp)
 {
     double c = model_cost(sp, sp.tau), more = 0.0;

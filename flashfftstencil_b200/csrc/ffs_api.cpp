@@ -181,7 +181,7 @@ struct ffs_plan {
     } dev[2];
     // wide tiles: a chunk's packed rows, and the twiddles per axis
     double2 *d_wide = nullptr;
-    double2 *d_wtw[3] = {nullptr, nullptr, nullptr};
+    double2 *d_wtw[2] = {nullptr, nullptr};
     double *d_frame = nullptr; // two buffers of the band's frame
     // direct steps: the launch of each pass kind, without its buffers
     LineWork line[2] = {};
@@ -463,7 +463,7 @@ struct PlanMemory {
 };
 
 // The spectra of a wide-tile plan, made on the device (`roots` per axis, in its memory).
-static cudaError_t wide_spectra(const ffs_plan *p, double2 *const roots[3])
+static cudaError_t wide_spectra(const ffs_plan *p, double2 *const roots[2])
 {
     const PlanSpec &sp = p->spec;
     cudaError_t e = cudaSuccess;
@@ -475,7 +475,7 @@ static cudaError_t wide_spectra(const ffs_plan *p, double2 *const roots[3])
         w.r = sp.radius;
         w.tau = sp.pass[k].tau;
         w.scale = sp.dim == 1 ? 1.0 : 0.5; // 2-D: the columns are twice the half spectra
-        for (int d = 0; d < 3; ++d) {
+        for (int d = 0; d < 2; ++d) {
             w.roots[d] = roots[d];
             w.tile[d] = sp.wtile[d];
             w.scale /= sp.wtile[d];
@@ -526,7 +526,7 @@ static ffs_status create_plan(ffs_plan **out, const ffs_problem *problem, Route 
     cudaError_t e;
     const PlanSpec &sp = p->spec;
     PlanMemory mem;
-    double2 *roots[3] = {nullptr, nullptr, nullptr};
+    double2 *roots[2] = {nullptr, nullptr};
     mem.put(&p->d_status, std::vector<int>{0});
     mem.put(&p->d_tables, sp.tables);
     mem.put(&p->d_aslices, sp.a_slices);
@@ -658,7 +658,7 @@ static WideWork wide_work(const ffs_plan *p, int kind, const double *src, double
     w.out = dst;
     w.work = p->d_wide;
     w.spec = p->dev[kind].spec;
-    for (int d = 0; d < 3; ++d) {
+    for (int d = 0; d < 2; ++d) {
         w.tw[d] = p->d_wtw[d];
         w.n[d] = sp.n[d];
         w.org[d] = ps.worg[d];

@@ -68,27 +68,27 @@ struct WideWork {
     const double *in;
     double *out;
     double2 *work;        // `chunk` tiles of packed rows
-    const double2 *spec;  // S^tau / (2 Nx Ny Nz), [kz][ky][kx], kx padded to Nx / 2 + 16
-    const double2 *tw[3]; // per axis: w_N^(m k1), then w_(N/16)^(m2 k2)
-    int64_t n[3], org[3], useful[3], vhi[3], nt[3];
+    const double2 *spec;  // S^tau / (2 Nx Ny), [ky][kx], kx padded to Nx / 2 + 16 (1-D: S^tau / N)
+    const double2 *tw[2]; // per axis, P points a thread: w_N^(m k1), then w_(N/P)^(m2 k2)
+    int64_t n[2], org[2], useful[2], vhi[2], nt[2];
     int64_t tile0;        // first tile of the chunk
     int ntiles;           // tiles of the chunk
-    int tile[3], halo[3];
+    int tile[2], halo[2];
     int periodic;
 };
 struct WideSpectrum {
     double2 *out;
     const double *weights;
-    const double2 *roots[3]; // exp(+2 pi i m / n) per axis, {re hi, re lo}, {im hi, im lo}
+    const double2 *roots[2]; // exp(+2 pi i m / n) per axis, {re hi, re lo}, {im hi, im lo}
     int dim, r, tau;
-    int tile[3];
+    int tile[2];
     double scale;
 };
 int wide_points(int n, int axis); // points per thread of a line of n (axis 0: rows, else columns)
 cudaError_t prepare_wide();
 cudaError_t launch_wide(const WideWork &w, int64_t tiles, int chunk, cudaStream_t s);
-size_t wide_tile_bytes(const int tile[3]);
-size_t wide_spectrum_count(const int tile[3]);
+size_t wide_tile_bytes(const int tile[2]);
+size_t wide_spectrum_count(const int tile[2]);
 cudaError_t launch_wide_spectrum(const WideSpectrum &p, cudaStream_t s);
 
 // 1D FP64 butterfly form (four-step DFT-4096 of radix-8 lines).

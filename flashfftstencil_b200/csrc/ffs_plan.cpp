@@ -662,13 +662,13 @@ double wide1_pass_cost(const PlanSpec &sp, const PassSpec &ps);
 
 // FFS_WIDE_TILE: "0" keeps wide tiles off, "512x1024" takes that edge wherever it fits.
 // Returns -1 off, 0 the model's choice, 1 forced.
-int wide_override(int dim, int tile[3])
+int wide_override(int dim, int tile[2])
 {
     const char *env = getenv("FFS_WIDE_TILE");
     if (!env || !*env)
         return 0;
-    int v[3] = {0, 0, 1};
-    const int got = sscanf(env, "%dx%dx%d", &v[0], &v[1], &v[2]);
+    int v[2] = {0, 0};
+    const int got = sscanf(env, "%dx%d", &v[0], &v[1]);
     if (got >= 1 && v[0] == 0)
         return -1;
     if (got != dim)
@@ -687,7 +687,7 @@ int wide_override(int dim, int tile[3])
 bool wide_geometry(const PlanSpec &sp, PassSpec *ps)
 {
     ps->nitems = 1;
-    for (int d = 0; d < 3; ++d) {
+    for (int d = 0; d < 2; ++d) {
         ps->whalo[d] = 0;
         ps->worg[d] = 0;
         ps->wuseful[d] = ps->wnt[d] = 1;
@@ -722,7 +722,7 @@ double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
 {
     if (sp.dim == 1)
         return wide1_pass_cost(sp, ps);
-    const double pts = (double)sp.wtile[0] * sp.wtile[1] * sp.wtile[2] * (double)ps.nitems;
+    const double pts = (double)sp.wtile[0] * sp.wtile[1] * (double)ps.nitems;
     const double chunks = std::ceil((double)ps.nitems / wide_chunk(sp, ps.nitems));
     const double tiles = pts * (wide_row_seconds(sp.wtile[0]) + wide_col_seconds(sp.wtile[1])) +
                          chunks * 3 * kWideLaunchSeconds;
@@ -782,7 +782,7 @@ double pick_wide1(PlanSpec *sp, int forced)
 double pick_wide(PlanSpec *sp)
 {
     double best = INFINITY;
-    int forced[3] = {0, 0, 1};
+    int forced[2] = {0, 0};
     const int mode = wide_override(sp->dim, forced);
     if (sp->form != FFS_FORM_FP64_FFT || sp->dim > 2 || sp->T == 0 || mode < 0)
         return best;

@@ -36,8 +36,8 @@ struct PassSpec {
     int64_t npx = 0, nitems = 0;
     // wide tiles (PlanSpec::wide): tile i of an axis covers worg + i * wuseful, its useful
     // cells start whalo cells in
-    int whalo[3] = {0, 0, 0};
-    int64_t worg[3] = {0, 0, 0}, wuseful[3] = {1, 1, 1}, wnt[3] = {1, 1, 1};
+    int whalo[2] = {0, 0};
+    int64_t worg[2] = {0, 0}, wuseful[2] = {1, 1}, wnt[2] = {1, 1};
 };
 
 struct PlanSpec {
@@ -53,7 +53,7 @@ struct PlanSpec {
     int slices = 0;
     int tile = 0;
     bool wide = false;           // wide tiles (ffs_wide.cu): `tile` is the x edge
-    int wtile[3] = {1, 1, 1};    // wide tile edges
+    int wtile[2] = {1, 1};       // wide tile edges
     int wchunk = 0;              // tiles per chunk of a wide pass (one workspace)
     bool direct = false;         // stepped directly, tau steps per pass, no transform:
     bool blocks = false;         // 2-D: by blocks (ffs_step.cu), else by marching warps (ffs_march.cu)

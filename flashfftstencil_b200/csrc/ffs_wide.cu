@@ -336,7 +336,8 @@ cudaError_t line_tiles(const WideWork &w, const BandWork &band, size_t band_smem
 //
 // S(k)^tau by repeated squaring multiplies the relative error of S by tau, so plain FP64
 // would lose log2(tau) bits where |S| is close to 1.  A double-double pair carries 106
-// bits; the roots come from the host in extended precision.
+// bits (sums by Knuth's and Dekker's error-free additions, products by a fused
+// multiply-add's exact remainder); the roots come from the host in extended precision.
 
 struct DD {
     double hi, lo;
@@ -383,31 +384,26 @@ __global__ void __launch_bounds__(256) spectrum_kernel(const WideSpectrum p)
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t line = i / H;
     const int kx = (int)(i - line * H);
-    if (line >= (int64_t)p.tile[1] * p.tile[2])
+    if (line >= p.tile[1])
         return;
     if (kx > p.tile[0] / 2) {
         p.out[i] = make_double2(0.0, 0.0);
         return;
     }
-    const int kz = (int)(line / p.tile[1]), ky = (int)(line - (int64_t)kz * p.tile[1]);
-    const int r = p.r, ry = p.dim >= 2 ? r : 0, rz = p.dim >= 3 ? r : 0, K = 2 * r + 1;
+    const int ky = (int)line, r = p.r, ry = p.dim == 2 ? r : 0, K = 2 * r + 1;
     const DD z0 = {0.0, 0.0};
     CDD s = {z0, z0};
-    for (int dz = -rz; dz <= rz; ++dz) {
-        CDD plane = {z0, z0};
-        for (int dy = -ry; dy <= ry; ++dy) {
-            CDD row = {z0, z0};
-            for (int dx = -r; dx <= r; ++dx) {
-                const double w = __ldg(p.weights + ((dz + rz) * (2 * ry + 1) + (dy + ry)) * K + (dx + r));
-                if (w != 0.0) {
-                    const CDD e = root_of(p.roots[0], p.tile[0], dx, kx);
-                    const DD wd = {w, 0.0};
-                    row = cdd_add(row, {dd_mul(e.re, wd), dd_mul(e.im, wd)});
-                }
+    for (int dy = -ry; dy <= ry; ++dy) {
+        CDD row = {z0, z0};
+        for (int dx = -r; dx <= r; ++dx) {
+            const double w = __ldg(p.weights + (dy + ry) * K + (dx + r));
+            if (w != 0.0) {
+                const CDD e = root_of(p.roots[0], p.tile[0], dx, kx);
+                const DD wd = {w, 0.0};
+                row = cdd_add(row, {dd_mul(e.re, wd), dd_mul(e.im, wd)});
             }
-            plane = cdd_add(plane, p.dim >= 2 ? cdd_mul(row, root_of(p.roots[1], p.tile[1], dy, ky)) : row);
         }
-        s = cdd_add(s, p.dim >= 3 ? cdd_mul(plane, root_of(p.roots[2], p.tile[2], dz, kz)) : plane);
+        s = cdd_add(s, p.dim == 2 ? cdd_mul(row, root_of(p.roots[1], p.tile[1], dy, ky)) : row);
     }
     CDD v = {{1.0, 0.0}, z0};
     for (int e = p.tau; e > 0; e >>= 1) {
@@ -528,14 +524,14 @@ cudaError_t launch_wide(const WideWork &w, int64_t tiles, int chunk, cudaStream_
 
 int wide_points(int n, int axis) { return axis == 0 ? wide::row_points(n) : wide::col_points(n); }
 
-size_t wide_tile_bytes(const int tile[3]) // workspace of one tile
+size_t wide_tile_bytes(const int tile[2]) // workspace of one tile
 {
-    return sizeof(double2) * (size_t)(tile[0] + 2 * wide::kPad) * (tile[1] / 2) * tile[2];
+    return sizeof(double2) * (size_t)(tile[0] + 2 * wide::kPad) * (tile[1] / 2);
 }
 
-size_t wide_spectrum_count(const int tile[3])
+size_t wide_spectrum_count(const int tile[2])
 {
-    return (size_t)(tile[0] / 2 + wide::kPad) * tile[1] * tile[2];
+    return (size_t)(tile[0] / 2 + wide::kPad) * tile[1];
 }
 
 cudaError_t launch_wide_spectrum(const WideSpectrum &p, cudaStream_t s)

@@ -1,17 +1,17 @@
 // FP64 butterfly form on wide tiles (256 .. 2048 cells per axis, a tile too large for one
-// SM's shared memory): the per-line pieces, host-callable where no exchange is involved.
+// SM's shared memory; 1024 .. 4096 in 1-D): the transform of one line.
 //
-// A line of N = 256 R3 points (R3 = 1, 2, 4, 8) is transformed by L = N / 16 threads holding
-// 16 points each, thread t points t + L a (a = 0..15):
-//   n = L n1 + m, m = R3 m1 + m2;  k = k1 + 16 k2 + 256 k3
-//   1. DFT-16 over n1 (thread m = t), times w_N^(m k1), put at (k1, m)
-//   2. get (k1, m2) = (t & 15, t >> 4) over m1, DFT-16, times w_L^(m2 k2), put back in place
-//   3. get (k1, k2) with k1 + 16 k2 = t + L g (g < 16 / R3) over m2, DFT-R3
-// Thread t then holds frequencies t + L a', a' = g + (16 / R3) k3: the layout of its input
+// A line of N = P P R3 points is transformed by L = N / P threads holding P points each,
+// thread t points t + L a (a = 0 .. P - 1).  P = 8 for rows of 256 and 512 and columns of 256,
+// else 16; R3 = 2, 4, 8 or 16.
+//   n = L n1 + m, m = R3 m1 + m2;  k = k1 + P k2 + P P k3
+//   1. DFT-P over n1 (thread m = t), times w_N^(m k1), put at (k1, m)
+//   2. get (k1, m2) = (t % P, t / P) over m1, DFT-P, times w_L^(m2 k2), put back in place
+//   3. get (k1, k2) with k1 + P k2 = t + L g (g < P / R3) over m2, DFT-R3
+// Thread t then holds frequencies t + L a', a' = g + (P / R3) k3: the layout of its input
 // points, so a forward transform feeds an inverse one with no reordering, and lanes on
-// consecutive t read and write consecutive points.  Two exchanges for every length (one for
-// N = 256): 16 points a thread moves half the shared-memory bytes per point that 8 would for
-// N = 1024 and 2048.
+// consecutive t read and write consecutive points.  Two exchanges for every length: with 8
+// points a thread the lines of 1024 and more would need a third.
 // Exchange slot of (k1, m): k1 * (L + 1) + m.  The odd pitch puts 8 consecutive k1 (steps 2
 // and 3) and 8 consecutive m (step 1) on distinct 16-byte bank groups; with C columns side by
 // side (slot * C + c) the same holds for every C that is a power of two.
@@ -61,8 +61,8 @@ __device__ __forceinline__ void twiddle(double &re, double &im, double2 w)
 }
 
 // One line's transform.  `sm`: the line's exchange slots (column c of C side by side: sm
-// already offset by c).  `tw`: w_N^(m k1) at k1 * L + m (k1 = 0..15), then w_L^(m2 k2) at
-// N + 16 m2 + k2.  `sync` makes the line's threads' shared-memory writes visible to each other.
+// already offset by c).  `tw`: w_N^(m k1) at k1 * L + m (k1 < P), then w_L^(m2 k2) at
+// N + P m2 + k2.  `sync` makes the line's threads' shared-memory writes visible to each other.
 template <int N, bool INV, int C, int P, class Sync>
 __device__ __forceinline__ void line_fft(double (&xr)[P], double (&xi)[P], int t, double2 *sm,
                                          const double2 *__restrict__ tw, Sync sync)

@@ -1568,7 +1568,8 @@ constexpr double kCopyBytesPerSecond = 48e9;
 // Fixed cost of one pass of a slab's sub-plan beyond the modelled tile waves:
 // launches, the band kernel's latency (about 30 us for tau = 8 whatever the box
 // count), and the first and last waves of a launch of a few hundred tiles.
-// Measured on Box2D9P slabs of 4096 x 192..1024 cells, tau 8.
+// Measured on Box2D9P slabs of 4096 x 192..1024 cells, tau 8.  Direct steps have no band, and their model has
+// the launch.
 constexpr double kSlabPassSeconds = 25e-6;
 constexpr int kMaxSlabs = 16;
 constexpr int64_t kMinSlabBytes = 4ll << 20;
@@ -1632,7 +1633,7 @@ SlabModel slab_model(const PlanSpec &sp)
             return false;
         out->count = kk;
         out->a = out->c = (double)h * row * sizeof(double) / kCopyBytesPerSecond;
-        out->b = ss.est_seconds + ss.passes * kSlabPassSeconds;
+        out->b = ss.est_seconds + (ss.direct ? 0.0 : ss.passes * kSlabPassSeconds);
         return true;
     };
     if (forced > 0) {

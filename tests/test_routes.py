@@ -124,3 +124,11 @@ def test_slab_passes_are_those_of_the_one_sm_tiles(edge, form, tmp_path):
                        timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == ["True", "True"]
+
+
+@pytest.mark.parametrize("shape,ext,T,slabs", [("Box3D27P", (200, 180, 160), 10, 4), ("Heat-3D", (200, 208, 170), 13, 3)])
+def test_host_slabs_of_direct_steps_are_not_charged_the_tiles_passes(shape, ext, T, slabs):
+    """A slab's pass of one direct step has no band to wait for: with the tiles' 25 us a pass these grids went in one
+    slab less or half of them (Box3D27P 1908 us, 1590 in four slabs, 1727 in four on the tiles)."""
+    info = ffs.describe(3, shape, ext, T, boundary="fixed", form="auto")
+    assert _direct(info) and info["host_slabs"] == slabs

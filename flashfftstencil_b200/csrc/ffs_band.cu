@@ -16,11 +16,11 @@ namespace band {
 
 constexpr int NT = 256;
 
-template <int DIM, int NTAPS, bool ROWS = false>
+template <int DIM, int NTAPS, bool ROWS = false, int WARPS = 1>
 __global__ void __launch_bounds__(NT) band_kernel(const BandWork p)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    process_box<DIM, NTAPS, ROWS>(p, blockIdx.x, smem, NT);
+    process_box<DIM, NTAPS, ROWS, WARPS>(p, blockIdx.x, smem, NT);
 }
 
 } // namespace band
@@ -33,6 +33,7 @@ cudaError_t prepare_band(size_t max_smem)
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
     };
     set((const void *)band::band_kernel<1, 0>);
+    set((const void *)band::band_kernel<1, 0, false, 2>);
     set((const void *)band::band_kernel<2, 0>);
     set((const void *)band::band_kernel<2, 5>);
     set((const void *)band::band_kernel<2, 9>);
@@ -49,7 +50,9 @@ cudaError_t launch_band(const BandWork &w, size_t smem_bytes, cudaStream_t s)
         return cudaSuccess;
     // stencils of 5 and 9 (2D: Heat-2D; Box2D9P, Star2D9P) and 7 and 27 (3D: Heat-3D, Box3D27P)
     // non-zero taps keep their taps in registers
-    if (w.dim == 1)
+    if (w.dim == 1 && band::warp_multiple(w) == 2)
+        band::band_kernel<1, 0, false, 2><<<w.nboxes, band::NT, smem_bytes, s>>>(w);
+    else if (w.dim == 1)
         band::band_kernel<1, 0><<<w.nboxes, band::NT, smem_bytes, s>>>(w);
     else if (w.dim == 2 && w.ntaps == 5)
         band::band_kernel<2, 5><<<w.nboxes, band::NT, smem_bytes, s>>>(w);

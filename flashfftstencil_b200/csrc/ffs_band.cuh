@@ -7,7 +7,14 @@
 namespace ffst {
 namespace band {
 
-constexpr int kWarpCells = 8; // cells per lane of the one-warp 1-D path
+constexpr int kWarpCells = 8; // cells per lane of the one-warp 1-D path, or twice as many
+
+// Multiples of 256 staged cells of a 1-D band's largest box that one warp steps: 2 where it takes 16 cells a lane,
+// else 1 (smaller boxes, and those that the block steps).
+__host__ __device__ inline int warp_multiple(const BandWork &p)
+{
+    return p.r >= 1 && p.r <= 4 && p.max_vol > 32 * kWarpCells && p.max_vol <= 64 * kWarpCells ? 2 : 1;
+}
 
 // One warp steps a 1-D box whose staged region [L, L + ext) has at most 32 * K cells,
 // entirely in registers: lane l holds cells [lK, lK + K), the R cells beyond each end
@@ -85,7 +92,10 @@ struct QuickDiv {
 // steps (weights and offsets otherwise come from shared memory at every tap of every step).
 // ROWS: 2-D 3 x 3 boxes may step by warp rows (below); a separate instantiation, since that
 // path's registers (64 against 48) cost the other boxes occupancy.
-template <int DIM, int NTAPS = 0, bool ROWS = false>
+// WARPS: one warp steps 1-D boxes of up to 256 WARPS staged cells.  The code of 16 cells a lane beside
+// it slowed the block's loop by 5 to 7 % (radius 7, 50000 cells, T = 100: 84 to 89 us), so bands without
+// such boxes take WARPS = 1.
+template <int DIM, int NTAPS = 0, bool ROWS = false, int WARPS = 2>
 __device__ __forceinline__ void process_box(const BandWork &p, int box, unsigned char *smem, int nthreads)
 {
     const BandBox bx = p.boxes[box];
@@ -95,18 +105,22 @@ __device__ __forceinline__ void process_box(const BandWork &p, int box, unsigned
         const int64_t lo = bx.lo[0] - rt < 0 ? 0 : bx.lo[0] - rt;
         const int64_t hi = bx.lo[0] + bx.ext[0] + rt > p.n[0] ? p.n[0] : bx.lo[0] + bx.ext[0] + rt;
         const int ext = (int)(hi - lo);
-        if (ext <= 64 * kWarpCells && r >= 1 && r <= 4) { // (8 cells a lane, or 16)
+        if (ext <= 32 * kWarpCells * WARPS && r >= 1 && r <= 4) { // (8 cells a lane, or 16)
             if (threadIdx.x < 32) {
-                const bool wide = ext > 32 * kWarpCells;
-                switch (wide ? r + 4 : r) {
+                if (WARPS > 1 && ext > 32 * kWarpCells) {
+                    switch (r) {
+                    case 1: process_box_1d_warp<1, WARPS * kWarpCells>(p, bx, lo, ext); break;
+                    case 2: process_box_1d_warp<2, WARPS * kWarpCells>(p, bx, lo, ext); break;
+                    case 3: process_box_1d_warp<3, WARPS * kWarpCells>(p, bx, lo, ext); break;
+                    default: process_box_1d_warp<4, WARPS * kWarpCells>(p, bx, lo, ext); break;
+                    }
+                    return;
+                }
+                switch (r) {
                 case 1: process_box_1d_warp<1, kWarpCells>(p, bx, lo, ext); break;
                 case 2: process_box_1d_warp<2, kWarpCells>(p, bx, lo, ext); break;
                 case 3: process_box_1d_warp<3, kWarpCells>(p, bx, lo, ext); break;
-                case 4: process_box_1d_warp<4, kWarpCells>(p, bx, lo, ext); break;
-                case 5: process_box_1d_warp<1, 2 * kWarpCells>(p, bx, lo, ext); break;
-                case 6: process_box_1d_warp<2, 2 * kWarpCells>(p, bx, lo, ext); break;
-                case 7: process_box_1d_warp<3, 2 * kWarpCells>(p, bx, lo, ext); break;
-                default: process_box_1d_warp<4, 2 * kWarpCells>(p, bx, lo, ext); break;
+                default: process_box_1d_warp<4, kWarpCells>(p, bx, lo, ext); break;
                 }
             }
             return;

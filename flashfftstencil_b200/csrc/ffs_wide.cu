@@ -252,9 +252,10 @@ template <int N>
 using LineShape = Shape<N, 16>;
 
 // (not inlined: inside the kernel its registers made the lines' code spill)
+template <int WARPS>
 __device__ __noinline__ void band_block(const BandWork &band, int box, unsigned char *smem)
 {
-    band::process_box<1>(band, box, smem, kLineThreads);
+    band::process_box<1, 0, false, WARPS>(band, box, smem, kLineThreads);
 }
 
 template <int N>
@@ -266,7 +267,11 @@ __global__ void __launch_bounds__(kLineThreads, 2) line_tiles_kernel(const __gri
     extern __shared__ __align__(16) double2 smem[];
     chain_wait();
     if ((int)blockIdx.x >= tile_blocks) {
-        band_block(band, (int)blockIdx.x - tile_blocks, reinterpret_cast<unsigned char *>(smem));
+        const int box = (int)blockIdx.x - tile_blocks;
+        if (band::warp_multiple(band) == 2)
+            band_block<2>(band, box, reinterpret_cast<unsigned char *>(smem));
+        else
+            band_block<1>(band, box, reinterpret_cast<unsigned char *>(smem));
         return;
     }
     const int l = threadIdx.x / S::L, t = threadIdx.x % S::L;

@@ -36,3 +36,22 @@ def test_staged_sizes(monkeypatch, radius, staged, past, in_place, offset):
     plan.run(d, out)
     torch.cuda.synchronize()
     assert rel_errors(out.cpu().numpy(), oracle.run(x, w, radius, T, oracle.FIXED))[0] <= TOL
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp64_fft"])
+@pytest.mark.parametrize("staged,past", [(256, 0), (256, 1), (512, 0), (512, 1)])
+@pytest.mark.parametrize("radius", [1, 4, 5])
+def test_staged_sizes_beside_one_sm_tiles(radius, staged, past, form):
+    """The band kernel's own launch, with the 4096-cell tile and the step count by name; radius 5 has no warp's path."""
+    import torch
+    n, tau = 9001, staged // (2 * radius) + past
+    T = 2 * tau + 1  # and a short last pass
+    w = seeded_weights(1, radius, 3)
+    plan = ffs.Plan(1, None, (n,), T, weights=w, radius=radius, boundary="fixed", form=form, tile=4096, tau=tau)
+    assert plan.info["tile"] == 4096 and plan.info["tau"] == tau
+    x = seeded_grid((n,), 4)
+    d = torch.from_numpy(x).cuda()
+    out = torch.full_like(d, float("nan"))
+    plan.run(d, out)
+    torch.cuda.synchronize()
+    assert rel_errors(out.cpu().numpy(), oracle.run(x, w, radius, T, oracle.FIXED))[0] <= TOL

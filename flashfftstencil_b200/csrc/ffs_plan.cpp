@@ -438,6 +438,7 @@ constexpr double kMarchLaunchSeconds = 5e-6; // launch, first rows
 constexpr double kMarchBytesPerSecond = 5e12;
 // 1-D: launch and copies; a step of a warp alone; multiply-adds with every SM busy
 constexpr double kLineLaunchSeconds = 6e-6, kLineStepSeconds = 0.04e-6, kLineCellSeconds = 1.5e-9;
+constexpr double kLineChainSeconds = 1.5e-6; // what a pass behind another does not wait for
 constexpr double kLineFmaPerSecond = 9e12;
 constexpr double kMarchRowSeconds = 0.13e-6; // a warp alone: one level of one row
 
@@ -484,32 +485,48 @@ double march3_cost(const PlanSpec &sp)
     return std::max(march3_units(&w, (int)sp.taps.size(), 148), 16.0 * (double)sp.cells / kMarchBytesPerSecond);
 }
 
+// 1-D: seconds of a step of the box at a fixed face, 2 r tau staged cells (measured on 7001 to 20000 cells, radius 1
+// to 8).  Up to radius 4 and 512 cells one warp steps it, 8 or 16 cells a lane.  Else a block does with a barrier per
+// step, 1024 cells at a time: radius 7, us a step, 0.85 in a launch of its own, as a block among line tiles 0.95
+// up to 1024 cells, 1.65 to 2048, 2.4 to 3072 and 3.2 above; radius 1, 2, 5 and 8 there 0.41, 0.51, 0.75 and 1.05.
+double box1_step(const PlanSpec &sp, int tau, bool among_lines)
+{
+    const int64_t staged = std::min<int64_t>(2ll * sp.radius * tau, sp.n[0]);
+    if (sp.boundary != FFS_BOUNDARY_FIXED || staged == 0 || (sp.open_faces & 3) == 3)
+        return 0.0;
+    if (sp.radius <= 4 && staged <= 512)
+        return staged <= 256 ? 0.03e-6 + 0.04e-6 * sp.radius : 0.06e-6 + 0.055e-6 * sp.radius;
+    const double chunk = (among_lines ? 0.046e-6 : 0.038e-6) * (double)sp.taps.size();
+    return (among_lines ? 0.27e-6 : 0.28e-6) + chunk * std::ceil((double)staged / 1024);
+}
+
 // The modelled solve on the form's one-SM tiles, to compare with the other routes.  Corrections to the
 // model that ranks the tiles' own step counts:
 // - 3-D: it counts 3 us per pair of 16^3 tiles (its band and launch terms were fitted with that), but a
 //   pair takes 6 us: 100 x 90 x 70, periodic, T = 10 81 us, 256^3 at T = 4 443 us;
 // - 2-D: an odd row length rules TMA out, and the 64 x 64 tiles of a 1999 x 2047 grid took 1.9 times as
 //   long with wrapped plain loads, 1.3 times with clipped ones;
-// - 1-D: a wave takes 10.5 us, not 6 (16.7 M cells 150 us, 44.3 M 404 us, a few thousand 14.8), and a band
-//   of short boxes hides beside it (2^20, fixed, T = 64: 14.9 us).  Boxes of 2 r tau staged cells are one warp's
-//   up to 512, but deeper ones than r tau = 85 were not timed beside these tiles: their band counts in full.
+// - 1-D: a wave takes 10.5 us, not 6 (16.7 M cells 150 us, 44.3 M 404 us, a few thousand 14.8), and the boxes are
+//   stepped beside the tiles (radius 7, 8 and 5, one pass of 18, 32 and 80 steps 18.4, 31.9 and 59.0 us).  The
+//   tiles that share their SMs are late: 4.8 M cells, radius 3, 140 steps 91 us (tiles 57, boxes 76), 9.8 M, radius
+//   5, 154 steps 274 us (140, 171), 2.1 M, radius 6, 65 steps 52 us (36, 51).
 double tile_route_cost(const PlanSpec &sp)
 {
     double c = model_cost(sp, sp.tau), more = 0.0;
     if (sp.form != FFS_FORM_FP64_FFT || !tile_holds(sp, sp.tau))
         return c;
+    PassSpec ps;
+    geometry(sp, sp.tau, &ps);
+    const double waves = std::ceil((double)ps.nitems / 148);
+    if (sp.dim == 1) {
+        const double tiles = waves * 10.5e-6 + 4e-6, boxes = sp.tau * box1_step(sp, sp.tau, false);
+        return sp.passes * std::max(tiles, boxes + 3e-6 + 0.8 * std::max(tiles - 25e-6, 0.0));
+    }
     if (sp.dim == 3 && sp.tile == 16)
         more = 3e-6;
     else if (sp.dim == 2 && sp.tile == 64 && (sp.n[0] & 1))
         more = 5.7e-6 * (sp.boundary == FFS_BOUNDARY_PERIODIC ? 0.9 : 0.3);
-    else if (sp.dim == 1)
-        more = 4.5e-6;
-    PassSpec ps;
-    geometry(sp, sp.tau, &ps);
-    c += sp.passes * std::ceil((double)ps.nitems / 148) * more;
-    if (sp.dim == 1 && ps.nitems > 0 && 3 * sp.radius * sp.tau <= 256)
-        c -= sp.passes * band_cost(sp, ps, 148);
-    return c;
+    return c + sp.passes * waves * more;
 }
 
 double pick_direct3(PlanSpec *sp, bool forced)
@@ -554,7 +571,9 @@ double pick_direct1(PlanSpec *sp, bool forced)
         if (most == 0)
             continue;
         even_steps(sp->T, most, 3, [&](int tau, int passes) {
-            const double c = passes * line_cost(*sp, k, tau);
+            // (a pass starts up while the one before it ends: radius 3, 17121 cells, three passes of 32 steps take
+            // 20.9 us, radius 2, 116920 cells, eight of 41 86.3)
+            const double c = passes * line_cost(*sp, k, tau) - (passes - 1) * kLineChainSeconds;
             if (c < best) {
                 best = c;
                 sp->line_k = k;
@@ -737,12 +756,13 @@ double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
 double wide1_pass_cost(const PlanSpec &sp, const PassSpec &ps)
 {
     const double waves = (double)ps.nitems * sp.wtile[0] / (148.0 * 16384);
-    double band = 0.0; // a box steps by one warp up to 512 staged cells, else by a block with a barrier per step
-    if (sp.boundary == FFS_BOUNDARY_FIXED)
-        band = ps.tau * (2.0 * sp.radius * ps.tau <= 512 ? 0.01e-6 + 0.06e-6 * sp.radius : 0.5e-6);
     // 2^20 cells at T = 64 10.6 us with 2048 (12.8 with 1024, 11.2 with 4096), 16.7 M at T = 32 87 (90, 92)
     const double edge = sp.wtile[0] == 1024 ? 1.08 : sp.wtile[0] == 4096 ? 1.04 : 1.0;
-    return std::max(edge * std::max(waves * kWide1WaveSeconds, kWide1LeastSeconds), band + 3e-6) + kWide1LaunchSeconds;
+    const double tiles = edge * std::max(waves * kWide1WaveSeconds, kWide1LeastSeconds);
+    // the boxes are the launch's last blocks: with more tiles than a wave they start with its last one (1.26 M
+    // cells, radius 2, 230 steps of 920 staged cells in 1024-cell tiles: 176 us a pass)
+    const double before = std::max(tiles - edge * kWide1LeastSeconds, 0.0);
+    return std::max(tiles, before + ps.tau * box1_step(sp, ps.tau, true)) + kWide1LaunchSeconds;
 }
 
 double pick_wide1(PlanSpec *sp, int forced)

@@ -132,3 +132,15 @@ def test_host_slabs_of_direct_steps_are_not_charged_the_tiles_passes(shape, ext,
     slab less or half of them (Box3D27P 1908 us, 1590 in four slabs, 1727 in four on the tiles)."""
     info = ffs.describe(3, shape, ext, T, boundary="fixed", form="auto")
     assert _direct(info) and info["host_slabs"] == slabs
+
+
+@pytest.mark.parametrize("form", ["auto", "fp64_fft"])
+@pytest.mark.parametrize("n,T,radius", [(3_416, 458, 7), (188_069, 134, 8), (893_929, 268, 7), (91_237, 1_838, 7),
+                                        (1_259_431, 1_146, 2), (2_437_720, 820, 3)])
+def test_lines_do_not_pay_for_deep_boxes_with_few_passes(n, T, radius, form):
+    """A block's step of the box at a face costs with its cells and taps (0.4 to 3.6 us, where 0.5 was modelled): boxes of
+    1600 to 3800 staged cells took 1.6 to 4 times as long as the one-SM tiles' solve (188069 cells, radius 8, T = 134
+    in one pass 335 us, in three 122)."""
+    w = np.full(2 * radius + 1, 1.0 / (2 * radius + 1))
+    info = ffs.describe(1, None, (n,), T, weights=w, radius=radius, boundary="fixed", form=form)
+    assert 2 * radius * info["tau"] <= 1024

@@ -336,22 +336,29 @@ void march_units(MarchWork *w, int r, bool star, int tau, int num_sms)
         all[i].first_unit = ring;
         area += (double)all[i].strips * (all[i].oy1 - all[i].oy0) * (ring ? 1.5 : 1.0);
     }
-    // rows per unit for the resident warps
+    // rows per unit for the resident warps: as few as leave no unit for a second wave (22 strips of 61 rows are 1188
+    // units of 3279 rows for 1184 warps: Heat-2D 2394 x 3279, periodic, tau 8 73 us a pass)
     constexpr int kLeastRows = 8; // (a launch of few rows is bound by its units' length: on the
                                   // frame of 1500 x 1300 at tau 4, 8 / 16 rows took 80 / 148 us in all)
-    const double rows = area / ((double)num_sms * march_warps(r, star, !w->periodic, tau));
-    w->units = 0;
+    const int slots = num_sms * march_warps(r, star, !w->periodic, tau);
     w->nregions = n;
-    for (int i = 0; i < n; ++i) {
-        MarchRegion &g = w->reg[i] = all[i];
-        const int total = g.oy1 - g.oy0;
-        int chunk = std::max((int)(g.first_unit ? rows / 1.5 : rows) + 1, kLeastRows);
-        const int parts = (total + chunk - 1) / chunk;
-        chunk = (total + parts - 1) / parts;
-        g.chunk = chunk;
-        g.first_unit = w->units;
-        w->units += g.strips * ((total + chunk - 1) / chunk);
-    }
+    auto split = [&](double rows) { // fills the regions, returns the units
+        int units = 0;
+        for (int i = 0; i < n; ++i) {
+            MarchRegion &g = w->reg[i] = all[i];
+            const int total = g.oy1 - g.oy0;
+            const int chunk = std::max((int)(all[i].first_unit ? rows / 1.5 : rows) + 1, kLeastRows);
+            const int parts = (total + chunk - 1) / chunk;
+            g.chunk = (total + parts - 1) / parts;
+            g.first_unit = units;
+            units += g.strips * ((total + g.chunk - 1) / g.chunk);
+        }
+        return units;
+    };
+    double rows = area / (double)slots;
+    w->units = split(rows);
+    for (int k = 0; k < 8 && w->units > slots && rows >= kLeastRows; ++k)
+        w->units = split(rows *= 1.01);
 }
 
 cudaError_t launch_march2d(const MarchWork &w, int r, bool star, int tau, cudaStream_t s)

@@ -430,17 +430,29 @@ int pick_tile(const PlanSpec &sp, int tau_override)
 
 // ---- direct stepping ----
 
-// Measured on 4096^2 and 1999 x 2047 grids (tau 1 .. 8, 5 to 25 taps): 9e12 multiply-adds per
-// second of the 18.4e12, strip and chunk margins counted, with three blocks per SM; the fixed
-// boundary's kernels and the deep ones, two per SM, have fewer warps to hide their latency.
-constexpr double kMarchFmaPerSecond = 9e12;
 constexpr double kMarchLaunchSeconds = 5e-6; // launch, first rows
-constexpr double kMarchBytesPerSecond = 5e12;
+constexpr double kMarchBytesPerSecond = 5e12, kMarchCachedBytesPerSecond = 7e12;
 // 1-D: launch and copies; a step of a warp alone; multiply-adds with every SM busy
 constexpr double kLineLaunchSeconds = 6e-6, kLineStepSeconds = 0.04e-6, kLineCellSeconds = 1.5e-9;
 constexpr double kLineChainSeconds = 1.5e-6; // what a pass behind another does not wait for
 constexpr double kLineFmaPerSecond = 9e12;
-constexpr double kMarchRowSeconds = 0.13e-6; // a warp alone: one level of one row
+
+// The marching kernel by radius, taps and boundary: seconds of a cell's step with every SM busy, margins counted, and of
+// one level of one row for a warp alone (300 x 260).  The first from 1500 x 1300 and 4130 x 5900, us, measured / model:
+// Heat-2D, periodic, tau 6 19.3 / 19.4 and 108 / 106, fixed, tau 4 17.5 / 16.9 and 108 / 103; Box2D9P, fixed, tau 4 21.7 /
+// 21.5 and 140 / 140; Star2D9P, fixed, tau 3 24.3 / 24.1 and 129 / 139; 25 taps, fixed, tau 2 25.8 / 25.2 and 158 / 167.
+struct MarchRate {
+    double cell, row;
+};
+MarchRate march_rate(int r, bool star, bool fixed, int tau)
+{
+    if (r == 1)
+        return star ? (fixed ? MarchRate{0.88e-12, 0.09e-6} : MarchRate{0.6e-12, 0.05e-6})
+                    : (fixed ? MarchRate{1.22e-12, 0.115e-6} : MarchRate{0.9e-12, 0.07e-6});
+    if (star)
+        return fixed ? MarchRate{tau == 4 ? 1.95e-12 : 1.6e-12, 0.195e-6} : MarchRate{1.15e-12, 0.13e-6};
+    return fixed ? MarchRate{tau == 1 ? 3.7e-12 : 3e-12, 0.33e-6} : MarchRate{2.5e-12, 0.21e-6};
+}
 
 // Modelled seconds of `tau` fused steps of one nx x ny region.
 double march_cost(const PlanSpec &sp, double nx, double ny, int tau)
@@ -448,23 +460,45 @@ double march_cost(const PlanSpec &sp, double nx, double ny, int tau)
     const int r = sp.radius;
     const bool fixed = sp.boundary == FFS_BOUNDARY_FIXED;
     const int warps = march_warps(r, sp.star, fixed, tau);
-    const double rate = kMarchFmaPerSecond * (warps == 12 ? (fixed ? 0.85 : 1.0) : (fixed ? 0.65 : 0.85));
+    const MarchRate rate = march_rate(r, sp.star, fixed, tau);
     const double U = march_width(r, tau), h = 2.0 * r * tau;
     const double strips = std::ceil(nx / U);
     const double rows = std::min(std::max(strips * ny / (148.0 * warps), 8.0), ny); // march_units
     const double cells = strips * 128 * ny * (rows + h) / rows;
-    const double latency = (rows + h) * tau * kMarchRowSeconds * (r == 1 ? 1.0 : 1.5);
-    return std::max(std::max(cells * tau * (double)sp.taps.size() / rate, latency),
-                    16.0 * nx * ny / kMarchBytesPerSecond) +
-           kMarchLaunchSeconds;
+    const double steps = cells * tau * rate.cell, latency = (rows + h) * tau * rate.row;
+    // grids of up to 100 MB, both counted, stay in L2 between passes, and part of them up to 300
+    const double moved = 16.0 * nx * ny, far = std::min(std::max((moved - 100e6) / 200e6, 0.0), 1.0);
+    const double bytes = moved / (kMarchCachedBytesPerSecond + far * (kMarchBytesPerSecond - kMarchCachedBytesPerSecond));
+    return std::max(std::max(steps, latency), bytes) + kMarchLaunchSeconds;
 }
 
-// One launch of the block kernel: a step of its tiles, one per SM at a time (5 taps 0.85 us,
-// 9 taps 1.05, 25 taps 1.8, measured on 300 x 260).
-double step_cost(const PlanSpec &sp, double tiles, int steps)
+// The block kernel's steps of its tiles, one per SM at a time (5 taps 0.85 us, 9 taps 1.05, 25 taps 1.8,
+// measured on 300 x 260).
+double step_seconds(const PlanSpec &sp, double tiles, int steps)
 {
-    const double one = (0.6 + 0.05 * (double)sp.taps.size()) * 1e-6;
-    return kMarchLaunchSeconds + steps * one * std::ceil(tiles / 148.0);
+    return steps * (0.6e-6 + 0.05e-6 * (double)sp.taps.size()) * std::ceil(tiles / 148.0);
+}
+
+// Its tiles of a grid (step_tiles: a tile at a fixed face has no margin there).
+double step_grid_tiles(const PlanSpec &sp, int steps)
+{
+    const double U = step_width(sp.radius, steps), H = sp.radius * steps;
+    double tiles = 1.0;
+    for (int d = 0; d < 2; ++d) {
+        const int walls = sp.boundary != FFS_BOUNDARY_FIXED ? 0
+                                                             : !(sp.open_faces >> 2 * d & 1) + !(sp.open_faces >> (2 * d + 1) & 1);
+        tiles *= std::max(std::ceil(((double)sp.n[d] - walls * H) / U), 1.0);
+    }
+    return tiles;
+}
+
+// One launch of it over a grid.  A tile is loaded and stored with nothing else on its SM: after the first, which
+// overlaps the launch, 2.7 us (4130 x 5900, one step of 44 to 47 tiles per SM, 5, 9 and 25 taps 162, 169 and 218 us).
+constexpr double kStepTileSeconds = 2.7e-6;
+double step_cost(const PlanSpec &sp, int steps)
+{
+    const double tiles = step_grid_tiles(sp, steps);
+    return kMarchLaunchSeconds + step_seconds(sp, tiles, steps) + kStepTileSeconds * (std::ceil(tiles / 148.0) - 1);
 }
 
 // FFS_DIRECT: "0" keeps direct stepping off, "march" or "blocks" takes that kernel wherever it
@@ -500,19 +534,25 @@ double box1_step(const PlanSpec &sp, int tau, bool among_lines)
     return (among_lines ? 0.27e-6 : 0.28e-6) + chunk * std::ceil((double)staged / 1024);
 }
 
+bool strips_win(const PlanSpec &sp);
+
 // The modelled solve on the form's one-SM tiles, to compare with the other routes.  Corrections to the
 // model that ranks the tiles' own step counts:
 // - 3-D: it counts 3 us per pair of 16^3 tiles (its band and launch terms were fitted with that), but a
 //   pair takes 6 us: 100 x 90 x 70, periodic, T = 10 81 us, 256^3 at T = 4 443 us;
-// - 2-D: an odd row length rules TMA out, and the 64 x 64 tiles of a 1999 x 2047 grid took 1.9 times as
-//   long with wrapped plain loads, 1.3 times with clipped ones;
+// - 2-D, 64 x 64: the tiles at a periodic face wrap with plain loads, and an odd row length rules TMA out for all (us,
+//   measured at 1, 2, 6, 14 and 34 waves: periodic 14.6, 27, 54, 98 to 103, 229, odd rows 16.5, -, 68, 168, 421;
+//   fixed 10.5, 21, 43, 89, -, odd rows 12.5, 21, -, 120, -).  A fixed boundary's boxes run beside the tiles: up to a
+//   depth of 8 cells 5.5 us of their modelled time do not show, to 14 3, then 2 (a band that is stepped on the frame
+//   shows as modelled), and 10 beside the longer 128 x 128 tiles.  One wave that leaves them few SMs may become two
+//   (25 taps, 752 x 885, T = 3, 136 tiles 16.9 or 24.7 us, 99 of them 10.6);
 // - 1-D: a wave takes 10.5 us, not 6 (16.7 M cells 150 us, 44.3 M 404 us, a few thousand 14.8), and the boxes are
 //   stepped beside the tiles (radius 7, 8 and 5, one pass of 18, 32 and 80 steps 18.4, 31.9 and 59.0 us).  The
 //   tiles that share their SMs are late: 4.8 M cells, radius 3, 140 steps 91 us (tiles 57, boxes 76), 9.8 M, radius
 //   5, 154 steps 274 us (140, 171), 2.1 M, radius 6, 65 steps 52 us (36, 51).
 double tile_route_cost(const PlanSpec &sp)
 {
-    double c = model_cost(sp, sp.tau), more = 0.0;
+    double c = model_cost(sp, sp.tau);
     if (sp.form != FFS_FORM_FP64_FFT || !tile_holds(sp, sp.tau))
         return c;
     PassSpec ps;
@@ -522,11 +562,28 @@ double tile_route_cost(const PlanSpec &sp)
         const double tiles = waves * 10.5e-6 + 4e-6, boxes = sp.tau * box1_step(sp, sp.tau, false);
         return sp.passes * std::max(tiles, boxes + 3e-6 + 0.8 * std::max(tiles - 25e-6, 0.0));
     }
+    if (sp.dim == 2 && ps.nitems > 0) {
+        const bool periodic = sp.boundary == FFS_BOUNDARY_PERIODIC, odd = sp.n[0] & 1;
+        const double items = (double)ps.nitems;
+        const double w = !periodic && items > 118 ? std::max(waves, 1.5) : waves;
+        double tiles;
+        if (sp.tile == 128)
+            tiles = 4e-6 + waves * kTile128Seconds;
+        else if (periodic)
+            tiles = odd ? 5e-6 + w * 11.9e-6 : std::min(w * 14.6e-6, 20e-6 + w * 5.75e-6);
+        else
+            tiles = odd ? 4.5e-6 + w * 8.2e-6 : w == 1 ? 10.5e-6 : 8e-6 + w * 5.75e-6;
+        const int depth = sp.radius * sp.tau;
+        double hidden = depth <= 8 ? 5.5e-6 : depth <= 14 ? 3e-6 : 2e-6;
+        if (sp.tile == 128)
+            hidden = waves > 1 || items <= 104 ? 10e-6 : 0.0;
+        else if (strips_win(sp))
+            hidden = 0.0;
+        return sp.passes * (tiles + std::max(band_cost(sp, ps, 148) - hidden, 0.0));
+    }
     if (sp.dim == 3 && sp.tile == 16)
-        more = 3e-6;
-    else if (sp.dim == 2 && sp.tile == 64 && (sp.n[0] & 1))
-        more = 5.7e-6 * (sp.boundary == FFS_BOUNDARY_PERIODIC ? 0.9 : 0.3);
-    return c + sp.passes * waves * more;
+        c += sp.passes * waves * 3e-6;
+    return c;
 }
 
 double pick_direct3(PlanSpec *sp, bool forced)
@@ -603,9 +660,10 @@ double pick_direct(PlanSpec *sp)
             continue;
         const int most = blocks ? step_max_steps(r) : march_max_tau(r, sp->star);
         even_steps(sp->T, most, 2, [&](int tau, int passes) {
-            const double U = blocks ? step_width(r, tau) : 1;
-            const double c = passes * (blocks ? step_cost(*sp, std::ceil(sp->n[0] / U) * std::ceil(sp->n[1] / U), tau)
-                                              : march_cost(*sp, (double)sp->n[0], (double)sp->n[1], tau));
+            auto pass = [&](int steps) {
+                return blocks ? step_cost(*sp, steps) : march_cost(*sp, (double)sp->n[0], (double)sp->n[1], steps);
+            };
+            const double c = (passes - 1) * pass(tau) + pass(sp->T - (passes - 1) * tau);
             if (c < best) {
                 best = c;
                 sp->blocks = blocks;
@@ -625,9 +683,7 @@ double direct_cost(const PlanSpec &sp, int tau)
         return line_cost(sp, sp.line_k, tau);
     if (sp.dim == 3)
         return march3_cost(sp);
-    const double U = step_width(sp.radius, tau);
-    return sp.blocks ? step_cost(sp, std::ceil(sp.n[0] / U) * std::ceil(sp.n[1] / U), tau)
-                     : march_cost(sp, (double)sp.n[0], (double)sp.n[1], tau);
+    return sp.blocks ? step_cost(sp, tau) : march_cost(sp, (double)sp.n[0], (double)sp.n[1], tau);
 }
 
 // The band of one wide pass, stepped on the frame: its seconds alone, and the share of them in
@@ -640,7 +696,7 @@ double frame_cost(const PlanSpec &sp, int tau, double *busy)
     const int most = frame_steps(sp), n = (tau + most - 1) / most, steps = (tau + n - 1) / n;
     const double U = step_width(sp.radius, steps), b = sp.radius * tau;
     const double tiles = 2.0 * ((double)sp.n[0] + (double)sp.n[1]) / U * std::ceil((1.5 * b - sp.radius * steps) / U);
-    const double launch = step_cost(sp, tiles, steps) - kMarchLaunchSeconds;
+    const double launch = step_seconds(sp, tiles, steps);
     *busy = n * launch * std::min(1.0, tiles / 148.0);
     return n * (launch + kMarchLaunchSeconds);
 }

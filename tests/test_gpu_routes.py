@@ -81,7 +81,7 @@ def test_the_first_line_of_a_process_has_its_kernel_loaded():
 
 def test_marching_units_fit_the_resident_warps(monkeypatch):
     """One unit per resident warp: with a fixed boundary's three regions of strips there were always some more, a second
-    wave (25 taps, one step: fixed 1.45 times the periodic time, 1.12 without it)."""
+    wave (25 taps, one step: fixed 1.6 times the periodic time, 1.12 without it)."""
     import torch
     monkeypatch.setenv("FFS_DIRECT", "march")
     nx, ny = 4130, 5800

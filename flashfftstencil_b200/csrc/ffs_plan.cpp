@@ -805,7 +805,11 @@ double wide_pass_cost(const PlanSpec &sp, const PassSpec &ps, int num_sms)
     // Box2D9P 1024^2 / 2048^2 / 4096^2 at T = 32 model 50 / 106 / 301 us, measured 46 / 113 / 303)
     double busy = 0.0;
     const double band = sp.frame ? frame_cost(sp, ps.tau, &busy) : (busy = band_cost(sp, ps, num_sms));
-    return std::max(tiles + 0.7 * busy, band);
+    // boxes of more cells than a block decodes once (2 x 1024) take several times their modelled work beside the tiles'
+    // small blocks (2802 x 1554, us, tiles alone / with the band: radius 3, 8 and 11 steps 78 / 198 and 89 / 313, radius
+    // 6, 3 steps 72 / 259, modelled work 55, 90 and 28)
+    const double share = !sp.frame && ps.band_max_vol > 2048 ? 3.0 : 0.7;
+    return std::max(tiles + share * busy, band);
 }
 
 // 1-D: seconds of one pass.  An SM holds 8192 complex points (16384 tile cells) at a time.

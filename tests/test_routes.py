@@ -163,3 +163,13 @@ def test_the_model_of_few_steps_holds_on_large_grids(shape, ext, T, boundary, us
 def test_small_fixed_grids_stay_on_one_sm_tiles(shape, ext, T):
     """fp64_fft by name, a single wave whose boxes run beside it: 9.0 and 10.6 us, on wide tiles 13.2 and 13.0."""
     assert ffs.describe(2, shape, ext, T, boundary="fixed", form="fp64_fft")["tile"] == 64
+
+
+@pytest.mark.parametrize("radius,ext,T", [(7, (874, 938), 33), (7, (1774, 1392), 3), (3, (314, 340), 6), (3, (1270, 916), 34)])
+def test_wide_tiles_do_not_take_deep_boxes_for_few_passes(radius, ext, T):
+    """From radius 3 on the band of a wide pass goes by boxes: past 2048 staged cells they took several times what was
+    modelled (radius 7, 874 x 938, T = 33 2728 us in eleven wide passes, 1250 on 64 x 64 tiles)."""
+    w = np.full((2 * radius + 1,) * 2, 1.0 / (2 * radius + 1) ** 2)
+    info = ffs.describe(2, None, ext, T, weights=w, radius=radius, boundary="fixed", form="fp64_fft")
+    depth = radius * info["tau"]
+    assert info["tile"] < 256 or 2 * depth * (32 + 2 * depth) <= 2048  # (a box at a face stages two depths of it)

@@ -2,7 +2,7 @@
 // down the rows.
 //
 // Where: short runs (few steps between two uses of a grid), where tau (2r+1)^2 multiply-adds
-// per cell cost less than two transforms (Star2D9P 1999 x 2047, T = 4: 64 x 64 tiles 82 us, this 39).
+// per cell cost less than two transforms (Star2D9P 1999 x 2047, T = 4: 64 x 64 tiles 82 us, this 34).
 //
 // A warp owns a strip of 32 K columns, K consecutive ones per lane, and reads the region's rows
 // in order.  Level s (0-based) turns row y of step s into row y - r of step s + 1: row y adds its
@@ -306,8 +306,8 @@ int march_max_tau(int r, bool star)
 int march_warps(int r, bool star, bool fixed, int tau) { return march::kWarps * march::blocks_per_sm(r, star, fixed, tau); }
 int march_width(int r, int tau) { return march::W - 2 * r * tau; }
 
-// Splits each region's output into strips and row chunks, one unit for every resident warp
-// (each unit re-reads 2 r tau rows of its neighbours, so chunks are as long as that allows).  With a
+// Splits a region's output (one region: with a fixed boundary it becomes up to three) into strips and row
+// chunks, one unit for every resident warp (each unit re-reads 2 r tau rows of its neighbours, so chunks are as long as that allows).  With a
 // fixed boundary the strips at the ring are regions of their own with shorter chunks: their
 // rows take about 1.5 times as long, and the launch ends with its longest unit.
 void march_units(MarchWork *w, int r, bool star, int tau, int num_sms)

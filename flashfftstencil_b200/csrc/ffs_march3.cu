@@ -2,8 +2,8 @@
 // z planes.
 //
 // Where: most 3-D runs.  The 16^3 tile's transforms keep (12 / 16)^3 = 0.42 of their points at two
-// fused steps: Box3D27P 512^3 takes 768 us a step that way, Heat-3D 740; one direct step 450 to 500 and 396
-// (HBM alone: 323).
+// fused steps: Box3D27P 512^3 takes 768 us a step that way, Heat-3D 740; one direct step 460 to 510 (the
+// more solves in a row, the longer) and 396 to 420 (HBM alone: 323).
 //
 // A block of 256 threads owns a 64 x 32 tile of a plane, a thread one column of kRows rows.  Planes (the
 // tile and one cell around it) come by cp.async into a ring in shared memory, kAhead planes early.  A
@@ -12,8 +12,8 @@
 // written out.  Pending planes change roles by unrolling the plane loop three times.  A cell's taps are
 // summed in the tap list's order (dz, dy, dx).
 // The fixed ring's cells keep their value by a select from the source plane's centre.
-// Bound: HBM (16 bytes a cell) with few taps; with 27 the FP64 pipe and issue (ncu at 256^3: pipe 44 %,
-// issue 58 %, no dominant stall).  Two steps a launch, the second level's source through shared memory,
+// Bound: HBM (16 bytes a cell) with few taps; with 27 the FP64 pipe and issue (counters at 256^3: pipe 48 %,
+// issue 58 %, HBM 56 % of the copy rate, no dominant stall).  Two steps a launch, the second level's source through shared memory,
 // took as long per step (Heat-3D 401, Box3D27P 570 us at 512^3): HBM traffic halves, but the margins, a
 // second barrier per plane and spills at 128 registers take it back.
 #include <cmath>
@@ -245,7 +245,7 @@ cudaError_t dispatch(const March3Work &w, bool star, cudaStream_t s)
 // 144 units of 6 planes 5.8 us a step, in 288 of 3 planes 7.8; but Box3D27P 512^3 in 128 units 667, in 1152
 // 453).  Measured, us a step,
 // Large / Small: Heat-3D 65 x 33 x 9 4.8 / 3.4, 100 x 90 x 70 6.2 / 5.8, 236 x 144 x 99 15.0 / 15.6, 256^3 57 / 60;
-// Box3D27P 100 x 90 x 70 7.5 / 7.1, 256^3 60 / 64; Large at 512^3, fixed, 413 and 453.
+// Box3D27P 100 x 90 x 70 7.5 / 7.1, 256^3 60 / 64; Large at 512^3, fixed, 413 and 453 (a first solve; up to 420 and 510 in a row).
 constexpr double kMarch3PlaneSeconds = 1.5e-6, kMarch3TapSeconds = 0.012e-6;
 constexpr double kMarch3SmallPlaneSeconds = 0.85e-6, kMarch3SmallTapSeconds = 0.007e-6;
 constexpr double kMarch3LaunchSeconds = 2e-6;

@@ -723,7 +723,7 @@ bool strips_win(const PlanSpec &sp)
 constexpr int kWideEdges[] = {256, 512, 1024, 2048};
 // Workspace of one chunk of tiles.  Fewer, larger launches win over a workspace that stays in
 // the 126 MB L2: Box2D25P 8192^2, T = 128, took 2297 / 2213 / 2018 / 1821 us with chunks of
-// 32 / 80 / 160 / 1000 MB (1661 since its columns go group by group), Box2D9P 4096^2 at T = 32 321 / 293 / 280 / 267 us.
+// 32 / 80 / 160 / 1000 MB (1720 since its columns go group by group), Box2D9P 4096^2 at T = 32 321 / 293 / 280 / 267 us.
 constexpr size_t kWideChunkBytes = (size_t)1 << 30;
 // Seconds per tile point of a pass: both row kernels by the x edge, the column kernel by the
 // y edge (measured on the two grids above), and per kernel its launch and first and last waves.

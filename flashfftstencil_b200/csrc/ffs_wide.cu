@@ -16,11 +16,12 @@
 //   rows_inv   two useful rows packed again, inverse FFT-Nx, cropped stores.
 // Every global access of a line's threads is to consecutive addresses, every exchange is
 // conflict-free (ffs_wide.cuh).
-// Bound: rows by HBM (rows_fwd 0.87 of the copy rate, rows_inv 0.72 to 0.78: Box2D9P 4096^2 at T = 32 in
-// 512 x 512 tiles 73 and 68 us); the columns (127 us, 0.48) by the sum of their loads, four exchanges
-// and stores, with 16 warps on an SM at 128 registers.  8 points a thread and twice the warps spill (49 us
-// against 44 a launch of fewer tiles).  Against the 128 x 128 tiles: that solve, fixed, 505 -> 298 us, Box2D25P
-// 8192^2, periodic, T = 128 12878 -> 1661.  Replaces rfft_2d (src/2D/rfft_2d/2d_rfft_1_async.cu:17-364)
+// Bound: rows by HBM (rows_fwd 0.87 of the copy rate, rows_inv 0.72 to 0.78: Box2D9P 4096^2, periodic, T = 32
+// in 100 tiles of 512 x 512 73 and 68 us); the columns (127 us, 0.48) by the sum of their loads, four exchanges
+// and stores, with 16 warps on an SM at 128 registers (of 9.5 cycles between two issues of a warp 3.8 wait for
+// global loads, 2.0 for shared memory; FP64 pipe 39 %).  8 points a thread and twice the warps spill (49 us
+// against 44 a launch of fewer tiles).  Against the 128 x 128 tiles: that grid with a fixed boundary (81 tiles)
+// 505 -> 296 us, Box2D25P 8192^2, periodic, T = 128 12878 -> 1720.  Replaces rfft_2d (src/2D/rfft_2d/2d_rfft_1_async.cu:17-364)
 // like the one-SM tiles do.
 #include "ffs_wide.cuh"
 
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(col_threads(N), col_blocks_per_sm(N)) cols_ker
     const int groups = hx / C + 1;
     // The tiles' blocks of one group of columns one after the other: they share its part of the spectrum,
     // which, from 16 MB on (2^20 points), the workspace streaming by takes out of L2 before the next tile
-    // needs it (2048 x 2048 tiles, Box2D25P 8192^2 at T = 128 1813 -> 1661 us; 1024 x 2048 2200 -> 2125).
+    // needs it (2048 x 2048 tiles, Box2D25P 8192^2 at T = 128 1813 -> 1720 us; 1024 x 2048 2200 -> 2125).
     // Below, tile by tile: adjacent segments then lie close in time (1024 x 512 and smaller 2 % faster).
     const bool by_group = N * hx >= 1 << 20;
     const int outer = by_group ? p.ntiles : groups, hi_index = blockIdx.x / outer, lo_index = blockIdx.x - hi_index * outer;

@@ -159,7 +159,11 @@ ffs_status ffs_plan_create(ffs_plan **out, const ffs_problem *problem);
  * that repeats the process's previous ffs_execute call (same plan, same buffers)
  * replays a CUDA graph of the pass sequence, captured on a private stream at the
  * first repeat (not while the plan is traced, nor inside a caller's stream
- * capture); the plan keeps the graphs of up to four buffer pairs. */
+ * capture); the plan keeps the graphs of up to four buffer pairs.  Inside a
+ * caller's capture the calls of one plan are ordered by the graph alone, and they
+ * use the plan's workspace (a wide-tile plan's also for a single pass): graphs
+ * that captured the same plan must not run at the same time, nor beside another
+ * execution of it. */
 ffs_status ffs_execute(const ffs_plan *plan, const double *d_in, double *d_out, void *stream);
 
 /* Same as ffs_execute with host buffers: copies in, runs, copies out and
